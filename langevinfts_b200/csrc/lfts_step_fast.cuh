@@ -175,6 +175,7 @@ __global__ void __launch_bounds__(NT) kf_plane_forward(GridPlan g, const lfts_st
     if (jb.active && !jb.active[jb.replica]) return;
     const int x = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     load_stw<C, N, NT>(stw, g.stw);
+    __syncthreads();  // the z transforms below are warp-private but read twiddles that other warps loaded
     const long long poff = (long long)x * N * N;
     const T *qin = (const T *)jb.in + s * jb.in_stride + poff;
     const T *fac = (const T *)jb.fac + poff;
