@@ -182,7 +182,9 @@ int lfts_autotune(lfts_ctx ctx, int njobs, int reps, char *report, size_t report
  * at creation, or lfts_autotune's choice.  No counterpart in the reference. */
 int lfts_step_impl(lfts_ctx ctx, char *name, size_t cap);
 /* Make name the context's step implementation ("register-64", "register-96",
- * "cubic", "generic"); an error when the context has no such implementation.
+ * "cubic", "generic", or "cluster-<n>": sweeps as one launch of n-CTA clusters,
+ * n = 1, 2, 4, 8 or 16); an error when the context has no such implementation.
+ * Named kernels other than "cluster-<n>" also run the sweeps step by step.
  * Not during a graph capture.  No counterpart in the reference. */
 int lfts_set_step_impl(lfts_ctx ctx, const char *name);
 /* Discrete chain: out = [fac *] F^-1[ b * F[in] ] with b = bond (half=0) or
@@ -192,6 +194,13 @@ int lfts_set_step_impl(lfts_ctx ctx, const char *name);
  * (CudaSolverPseudo.cu:451-476); (half=1, with_fac=1) is the junction start of
  * CpuComputationDiscrete.cpp:402-445 fused into one pass. */
 int lfts_step_discrete(lfts_ctx ctx, const lfts_step_job *jobs, int njobs, int s, int half, int with_fac);
+/* Steps s0 .. s0 + nsteps - 1 of lfts_step_continuous / lfts_step_discrete for
+ * every job, where step s + 1 starts from what step s wrote (out of step s is
+ * in of step s + 1).  On grids small enough for the shared memory of a
+ * thread-block cluster all steps are one launch; otherwise the steps run one
+ * after the other.  No counterpart in the reference. */
+int lfts_sweep_continuous(lfts_ctx ctx, const lfts_step_job *jobs, int njobs, int s0, int nsteps);
+int lfts_sweep_discrete(lfts_ctx ctx, const lfts_step_job *jobs, int njobs, int s0, int nsteps, int half, int with_fac);
 
 /* ---- junctions and initial slices --------------------------------------- */
 

@@ -60,6 +60,8 @@ _SIGS = {
     "lfts_field_factors_batch": [C.c_void_p, C.c_void_p, C.c_double, C.c_void_p, C.c_int],
     "lfts_step_continuous": [C.c_void_p, C.c_void_p, C.c_int, C.c_int],
     "lfts_step_discrete": [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int],
+    "lfts_sweep_continuous": [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int],
+    "lfts_sweep_discrete": [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int],
     "lfts_junctions": [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p],
     "lfts_dots": [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p],
     "lfts_dots_static": [C.c_int, C.c_longlong, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p],

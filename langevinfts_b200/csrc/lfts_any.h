@@ -21,6 +21,12 @@ void any_step_discrete(const AnyGrid *a, cudaStream_t st, const lfts_step_job *j
 void any_planes_forward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj);
 void any_xpass_forward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj);
 
+// stress: x-transform of both zy spectra of a job and the weighted sums over k;
+// partials[(job * tiles + tile) * 3 + axis]
+int any_stress_tiles(const AnyGrid *a, int nj);
+void any_xstress(const AnyGrid *a, cudaStream_t st, const lfts_step_job *sj, const lfts_stress_job *jobs, int nj,
+                 const double *basis, double *partials);
+
 // CTAs per job of the cluster sweep for nj jobs; 0: the grid does not fit or the
 // separate passes are faster.  force: 0 by that rule, else this cluster size where it fits.
 int any_sweep_size(const AnyGrid *a, bool continuous, int nj, int force);

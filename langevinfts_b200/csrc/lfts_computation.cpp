@@ -532,16 +532,15 @@ void GpuComputation::enqueue_propagation() {
                                         (const void *const *)(base + L.deps), (const double *)(base + L.wts)));
                 break;
             case 1:
-                for (int s = 0; s < L.nsteps; s++) {
-                    if (realspace_)
-                        check_rc(lfts_step_realspace(ctx_, (const lfts_step_job *)(base + L.jobs), L.njobs, s, cb_->get_dim()));
-                    else
-                        check_rc(lfts_step_continuous(ctx_, (const lfts_step_job *)(base + L.jobs), L.njobs, s));
+                if (!realspace_) {
+                    check_rc(lfts_sweep_continuous(ctx_, (const lfts_step_job *)(base + L.jobs), L.njobs, 0, L.nsteps));
+                    break;
                 }
+                for (int s = 0; s < L.nsteps; s++)
+                    check_rc(lfts_step_realspace(ctx_, (const lfts_step_job *)(base + L.jobs), L.njobs, s, cb_->get_dim()));
                 break;
             case 2:
-                for (int s = 0; s < L.nsteps; s++)
-                    check_rc(lfts_step_discrete(ctx_, (const lfts_step_job *)(base + L.jobs), L.njobs, s, L.half, L.with_fac));
+                check_rc(lfts_sweep_discrete(ctx_, (const lfts_step_job *)(base + L.jobs), L.njobs, 0, L.nsteps, L.half, L.with_fac));
                 break;
             case 3:
                 check_rc(lfts_memcpy_d2d_async(ctx_, L.dst, L.src, L.bytes));

@@ -16,6 +16,8 @@
 #include "lfts_step_r8.cuh"
 #include "lfts_step_r12.cuh"
 #include "lfts_realspace.cuh"
+#include "lfts_reduce.cuh"
+#include "lfts_any.h"
 
 using namespace lfts;
 
@@ -51,6 +53,8 @@ struct lfts_ctx_s {
     int fast_ok = 0, r8_ok = 0, r12_ok = 0;  // families set up at creation (lfts_set_step_impl)
     int r12 = 0;              // 96^3: register-resident 12x8 plane kernels (lfts_step_r12.cuh)
     int nsm = 0;              // streaming multiprocessors of the device
+    AnyGrid *any = nullptr;   // any-extent kernels (NULL: a plane does not fit them, k_* serve)
+    int sweep = 0;            // cluster sweeps: 0 by rule, -1 never, n > 0 with n CTAs a job where that fits
     int xcap = 0;             // CTAs per SM of the persistent x-passes (0: the kernel's own residency)
     void *stw = nullptr;
     size_t sm_pf1 = 0, sm_pf2 = 0, sm_mid = 0, sm_inv1 = 0, sm_inv2 = 0, sm_x1 = 0, sm_x2 = 0;
@@ -237,6 +241,10 @@ template <typename T> static int setup_plan(lfts_ctx c) {
                     " does not fit in shared memory (" + std::to_string(c->sm_mid) + " > " + std::to_string(max_smem) + " bytes)");
     c->nbr2 = (int)c->sm_pf2 <= max_smem && (int)c->sm_x2 <= max_smem;
     CK((c->gen ? set_attrs_t<T, true>(max_smem) : set_attrs_t<T, false>(max_smem)));
+    if (g.M > 1) {  // Anderson mixing's contexts have one point and no transforms
+        c->any = any_create((int)sizeof(T), n, c->nsm, max_smem, err);
+        if (!c->any && !err.empty()) return fail(err);
+    }
     g.stw = nullptr;
     if (g.n0 == g.n1 && g.n1 == g.n2 && !std::getenv("LFTS_NO_FAST")) {
         const int N = g.n0;
@@ -330,6 +338,7 @@ extern "C" int lfts_ctx_destroy(lfts_ctx c) {
     cudaSetDevice(c->device);
     if (c->tables) cudaFree(c->tables);
     if (c->stw) cudaFree(c->stw);
+    any_destroy(c->any);
     if (c->partials) cudaFree(c->partials);
     if (c->sjobs) cudaFree(c->sjobs);
     if (c->sjobs_host) cudaFreeHost(c->sjobs_host);
@@ -719,6 +728,12 @@ extern "C" int lfts_step_continuous(lfts_ctx c, const lfts_step_job *jobs, int n
         c->launches += 5;
         return c->prec == 8 ? step_fast_dispatch<double>(c, jobs, nj, s, 0, 0, 0) : step_fast_dispatch<float>(c, jobs, nj, s, 0, 0, 0);
     }
+    if (c->any) {
+        c->launches += 5;
+        any_step_continuous(c->any, c->stream, jobs, nj, s);
+        CKLAUNCH();
+        return 0;
+    }
     c->launches += c->nbr2 ? 5 : 8;
     if (c->prec == 8) return c->gen ? step_cont_t<double, true>(c, jobs, nj, s) : step_cont_t<double, false>(c, jobs, nj, s);
     return c->gen ? step_cont_t<float, true>(c, jobs, nj, s) : step_cont_t<float, false>(c, jobs, nj, s);
@@ -744,9 +759,54 @@ extern "C" int lfts_step_discrete(lfts_ctx c, const lfts_step_job *jobs, int nj,
     if (c->fastN)
         return c->prec == 8 ? step_fast_dispatch<double>(c, jobs, nj, s, 1, half, with_fac)
                             : step_fast_dispatch<float>(c, jobs, nj, s, 1, half, with_fac);
+    if (c->any) {
+        any_step_discrete(c->any, c->stream, jobs, nj, s, half, with_fac);
+        CKLAUNCH();
+        return 0;
+    }
     if (c->prec == 8)
         return c->gen ? step_disc_t<double, true>(c, jobs, nj, s, half, with_fac) : step_disc_t<double, false>(c, jobs, nj, s, half, with_fac);
     return c->gen ? step_disc_t<float, true>(c, jobs, nj, s, half, with_fac) : step_disc_t<float, false>(c, jobs, nj, s, half, with_fac);
+}
+
+// ---------------------------------------------------------------- sweeps
+// CTAs per job of a cluster sweep, 0 for step by step.  The cubic and register families
+// keep their grids: 22 us a step at 32^3 FP64 against 32 in clusters of 16, 19 against 19 at 16^3.
+static int sweep_size(lfts_ctx c, bool continuous, int nj) {
+    if (!c->any || c->sweep < 0 || (c->sweep == 0 && c->fastN)) return 0;
+    return any_sweep_size(c->any, continuous, nj, c->sweep);
+}
+extern "C" int lfts_sweep_continuous(lfts_ctx c, const lfts_step_job *jobs, int nj, int s0, int nsteps) {
+    if (!c || !jobs) return fail("null argument");
+    if (nj <= 0 || nsteps <= 0) return 0;
+    if (nj > 65535) return fail("too many jobs in one launch (max 65535)");
+    const int cs = sweep_size(c, true, nj);
+    if (cs) {
+        CK((cudaError_t)any_sweep_continuous(c->any, c->stream, jobs, nj, s0, nsteps, cs));
+        c->launches += 1;
+        return 0;
+    }
+    for (int s = s0; s < s0 + nsteps; s++) {
+        const int rc = lfts_step_continuous(c, jobs, nj, s);
+        if (rc) return rc;
+    }
+    return 0;
+}
+extern "C" int lfts_sweep_discrete(lfts_ctx c, const lfts_step_job *jobs, int nj, int s0, int nsteps, int half, int with_fac) {
+    if (!c || !jobs) return fail("null argument");
+    if (nj <= 0 || nsteps <= 0) return 0;
+    if (nj > 65535) return fail("too many jobs in one launch (max 65535)");
+    const int cs = sweep_size(c, false, nj);
+    if (cs) {
+        CK((cudaError_t)any_sweep_discrete(c->any, c->stream, jobs, nj, s0, nsteps, half ? 1 : 0, with_fac ? 1 : 0, cs));
+        c->launches += 1;
+        return 0;
+    }
+    for (int s = s0; s < s0 + nsteps; s++) {
+        const int rc = lfts_step_discrete(c, jobs, nj, s, half, with_fac);
+        if (rc) return rc;
+    }
+    return 0;
 }
 
 // ---------------------------------------------------------------- junctions
@@ -786,71 +846,6 @@ extern "C" int lfts_junctions(lfts_ctx c, const lfts_junction_job *jobs, int nj,
 }
 
 // ---------------------------------------------------------------- reductions
-// warp + block sum of a double (block of NTHR threads); result valid in thread 0
-__device__ __forceinline__ double block_sum(double v, double *sh) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[w] = v;
-    __syncthreads();
-    v = 0;
-    if (w == 0) {
-        v = lane < NWARP ? sh[lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    }
-    return v;
-}
-
-// Compensated (error-free transform) summation for the FP32 propagator form:
-// sums of FP32 products are accumulated in FP64 as a pair (s, c) where s is
-// the running sum and c the running sum of the rounding errors of every
-// addition (Knuth's two-sum; Neumaier's improvement of Kahan's method), and
-// reduced across threads with the same transform.  The FP64 form keeps the
-// plain FP64 sums.
-__device__ __forceinline__ void comp_add(double &s, double &c, double x) {
-    const double t = s + x;
-    const double bp = t - s;
-    c += (s - (t - bp)) + (x - bp);
-    s = t;
-}
-// block sum of compensated pairs (block of NTHR threads, sh holds 2 * NWARP
-// doubles); s + c of the block is valid in thread 0
-__device__ __forceinline__ double block_sum_comp(double s, double c, double *sh) {
-    for (int o = 16; o > 0; o >>= 1) {
-        const double so = __shfl_down_sync(0xffffffffu, s, o), co = __shfl_down_sync(0xffffffffu, c, o);
-        comp_add(s, c, so);
-        c += co;
-    }
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) { sh[w] = s; sh[NWARP + w] = c; }
-    __syncthreads();
-    s = 0.0;
-    c = 0.0;
-    if (w == 0) {
-        s = lane < NWARP ? sh[lane] : 0.0;
-        c = lane < NWARP ? sh[NWARP + lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) {
-            const double so = __shfl_down_sync(0xffffffffu, s, o), co = __shfl_down_sync(0xffffffffu, c, o);
-            comp_add(s, c, so);
-            c += co;
-        }
-    }
-    return s + c;
-}
-template <typename T>
-struct Acc {  // plain FP64 sum for T = double, compensated FP64 sum for T = float
-    double s = 0.0, c = 0.0;
-    __device__ __forceinline__ void add(double x) {
-        if (sizeof(T) == 4) comp_add(s, c, x);
-        else s += x;
-    }
-    __device__ __forceinline__ double value() const { return s + c; }
-    __device__ __forceinline__ double block(double *sh) const {
-        return sizeof(T) == 4 ? block_sum_comp(s, c, sh) : block_sum(s, sh);
-    }
-};
-
 constexpr int DOT_CHUNKS = 128;
 
 template <typename T>
@@ -1014,11 +1009,17 @@ static int stress_t(lfts_ctx c, const lfts_stress_job *jobs, int nj, const doubl
     for (int j0 = 0; j0 < nj; j0 += max_chunk) {
         const int n = nj - j0 < max_chunk ? nj - j0 : max_chunk;
         if (2 * n > c->sjobs_cap) return fail("stress chunk too large");
-        if ((size_t)n * c->ntiles * 3 > c->partials_cap) return fail("stress chunk exceeds the partial-sum workspace");
+        const int ntiles = c->any ? any_stress_tiles(c->any, n) : c->ntiles;
+        if ((size_t)n * ntiles * 3 > c->partials_cap) return fail("stress chunk exceeds the partial-sum workspace");
         k_stress_prep<T><<<(n + 127) / 128, 128, 0, st>>>(jobs + j0, n, spec, g.Mc, c->sjobs);
-        k_plane_forward<T, 1, GEN><<<dim3(g.n0, 2 * n), NTHR, c->sm_pf1, st>>>(g, c->sjobs, 0, FM_NONE, 0, 0, c->zb);
-        k_xstress<T, GEN><<<dim3(c->ntiles, n), NTHR, smx, st>>>(g, c->sjobs, jobs + j0, basis, c->TJ, c->partials);
-        k_finish<T><<<dim3(n, 3), NTHR, 0, st>>>(c->partials, c->ntiles, (const double *)&jobs[j0].weight,
+        if (c->any) {
+            any_planes_forward(c->any, st, c->sjobs, 2 * n);
+            any_xstress(c->any, st, c->sjobs, jobs + j0, n, basis, c->partials);
+        } else {
+            k_plane_forward<T, 1, GEN><<<dim3(g.n0, 2 * n), NTHR, c->sm_pf1, st>>>(g, c->sjobs, 0, FM_NONE, 0, 0, c->zb);
+            k_xstress<T, GEN><<<dim3(c->ntiles, n), NTHR, smx, st>>>(g, c->sjobs, jobs + j0, basis, c->TJ, c->partials);
+        }
+        k_finish<T><<<dim3(n, 3), NTHR, 0, st>>>(c->partials, ntiles, (const double *)&jobs[j0].weight,
                                                 (int)sizeof(lfts_stress_job), 1.0, out + 3 * (long long)j0, 3, 3);
     }
     CKLAUNCH();
@@ -1211,7 +1212,10 @@ extern "C" int lfts_fft_forward(lfts_ctx c, const lfts_step_job *jobs, int nj) {
     if (nj > 65535) return fail("too many jobs in one launch (max 65535)");
     const GridPlan &g = c->g;
     const dim3 gp(g.n0, nj), gx(c->ntiles, nj);
-    if (c->gen) {
+    if (c->any) {
+        any_planes_forward(c->any, c->stream, jobs, nj);
+        any_xpass_forward(c->any, c->stream, jobs, nj);
+    } else if (c->gen) {
         k_plane_forward<double, 1, true><<<gp, NTHR, c->sm_pf1, c->stream>>>(g, jobs, 0, FM_NONE, 0, 0, c->zb);
         k_xpass_forward<double, true><<<gx, NTHR, c->sm_x1, c->stream>>>(g, jobs, 0, c->TJ);
     } else {
@@ -1495,8 +1499,16 @@ extern "C" int lfts_set_step_impl(lfts_ctx c, const char *name) {
         c->r8 = r8;
         c->r12 = r12;
         c->xcap = 0;
+        c->sweep = -1;  // the named kernels, step by step
         return 0;
     };
+    if (n.rfind("cluster-", 0) == 0 && c->any) {
+        const int cs = std::atoi(n.c_str() + 8);
+        if (any_sweep_size(c->any, true, 1, cs) != cs && any_sweep_size(c->any, false, 1, cs) != cs)
+            return fail("step implementation \"" + n + "\" is not available for this context");
+        c->sweep = cs;
+        return 0;
+    }
     if (n == "register-64" && c->r8_ok) return set(fastN, 1, 0);
     if (n == "register-96" && c->r12_ok) return set(fastN, 0, 1);
     if (n == "cubic" && fastN) return set(fastN, 0, 0);

@@ -31,11 +31,16 @@ constexpr int MAX_REG_RADIX = 16;
 __host__ __device__ __forceinline__ unsigned div_mul(unsigned d) { return d <= 1 ? 0u : (unsigned)(0x100000000ull / d + 1); }
 __device__ __forceinline__ int fdiv(int t, unsigned mul) { return mul ? (int)__umulhi((unsigned)t, mul) : t; }
 
-// one axis; radix[] is outermost-first: n = radix[0] * ... * radix[nf-1]
+// One axis, outermost radix first: n = radix[0] * ... * radix[nf-1].  Everything a
+// stage needs that the host can divide is divided there.
+struct Stage {
+    int radix, span;    // span: product of the radices inside this one
+    unsigned span_mul;  // division by the span
+    int nbf, twstep;    // butterflies a line, n / (span * radix)
+};
 struct Axis {
     int n, nf;
-    int radix[MAXF];
-    unsigned span_mul[MAXF];  // division by the span of the stage (product of the radices inside it)
+    Stage st[MAXF];
 };
 
 // The grid as the kernels see it: x-planes of n1 x n2 points (n2 fastest).  A
@@ -195,27 +200,25 @@ template <typename C> __device__ __forceinline__ C swap_ri(C v) {
     return r;
 }
 
-// One stage of radix R over all lines (span m).  The inverse transform is the
-// forward one of the values with real and imaginary parts exchanged.
+// One stage of radix R over all lines.  The inverse transform is the forward one
+// of the values with real and imaginary parts exchanged.
 template <int R, bool INV, typename C>
-__device__ __forceinline__ void stage(C *buf, const Lines &ln, int n, int m, unsigned m_mul, const C *tw) {
-    const int total = ln.nl * (n / R), ms = m * ln.es;
-    const int twstep = n / (m * R);
+__device__ __forceinline__ void stage(C *buf, const Lines &ln, const Stage &sg, const C *tw) {
+    const int total = ln.nl * sg.nbf, m = sg.span, ms = m * ln.es;
     for (int t = threadIdx.x; t < total; t += blockDim.x) {
         const int b = fdiv(t, ln.nl_mul), l = t - b * ln.nl;
-        const int blk = fdiv(b, m_mul), k1 = b - blk * m;
+        const int blk = fdiv(b, sg.span_mul), k1 = b - blk * m;
         C *p = buf + ln.off(l) + (blk * m * R + k1) * ln.es;
         C a[R];
 #pragma unroll
         for (int j = 0; j < R; j++) a[j] = INV ? swap_ri(p[j * ms]) : p[j * ms];
-        if (!INV && k1) {
-            const int e = k1 * twstep;
+        const int e = k1 * sg.twstep;
+        if (!INV && e) {
 #pragma unroll
             for (int j = 1; j < R; j++) a[j] = cmul(a[j], tw[j * e]);
         }
         dft<R>(a);
-        if (INV && k1) {
-            const int e = k1 * twstep;
+        if (INV && e) {
 #pragma unroll
             for (int j = 1; j < R; j++) a[j] = cmul(a[j], tw[j * e]);
         }
@@ -228,10 +231,11 @@ __device__ __forceinline__ void stage(C *buf, const Lines &ln, int n, int m, uns
 // sums output k of the pair (k, R - k), k = 0 .. (R-1)/2; all threads of a chunk
 // have read when the first writes.
 template <bool INV, typename C>
-__device__ void stage_prime(C *buf, const Lines &ln, int R, int n, int m, unsigned m_mul, const C *tw) {
+__device__ void stage_prime(C *buf, const Lines &ln, const Stage &sg, const C *tw) {
     using T = decltype(buf[0].x);
-    const int nbf = ln.nl * (n / R), ms = m * ln.es, H = (R - 1) / 2;
-    const int twstep = n / (m * R), wstep = n / R;
+    const int R = sg.radix, m = sg.span, twstep = sg.twstep, wstep = sg.nbf;
+    const unsigned m_mul = sg.span_mul;
+    const int nbf = ln.nl * sg.nbf, ms = m * ln.es, H = (R - 1) / 2;
     const int per = blockDim.x / (H + 1) < 1 ? 1 : blockDim.x / (H + 1);
     auto twiddle = [&]() {  // elementwise, over the inputs (forward) or the outputs (inverse)
         if (m == 1) return;
@@ -285,35 +289,31 @@ __device__ void stage_prime(C *buf, const Lines &ln, int R, int n, int m, unsign
     if (INV) twiddle();
 }
 
+template <bool INV, typename C>
+__device__ __noinline__ void run_stage(C *buf, const Lines ln, const Stage sg, const C *tw) {
+    switch (sg.radix) {
+        case 2: stage<2, INV>(buf, ln, sg, tw); break;
+        case 3: stage<3, INV>(buf, ln, sg, tw); break;
+        case 4: stage<4, INV>(buf, ln, sg, tw); break;
+        case 5: stage<5, INV>(buf, ln, sg, tw); break;
+        case 6: stage<6, INV>(buf, ln, sg, tw); break;
+        case 7: stage<7, INV>(buf, ln, sg, tw); break;
+        case 8: stage<8, INV>(buf, ln, sg, tw); break;
+        case 9: stage<9, INV>(buf, ln, sg, tw); break;
+        case 10: stage<10, INV>(buf, ln, sg, tw); break;
+        case 11: stage<11, INV>(buf, ln, sg, tw); break;
+        case 12: stage<12, INV>(buf, ln, sg, tw); break;
+        case 13: stage<13, INV>(buf, ln, sg, tw); break;
+        case 16: stage<16, INV>(buf, ln, sg, tw); break;
+        default: stage_prime<INV>(buf, ln, sg, tw); break;
+    }
+    __syncthreads();
+}
+
 // All stages of an axis over all lines; ends with a block barrier.
 template <bool INV, typename C>
-__device__ __noinline__ void transform(C *buf, const Lines ln, const Axis &ap, const C *tw) {
-    if (ap.nf == 0 || ln.nl == 0) return;
-    int m = INV ? ap.n : 1;
-    for (int i = 0; i < ap.nf; i++) {
-        const int f = INV ? i : ap.nf - 1 - i;
-        const int R = ap.radix[f];
-        if (INV) m /= R;
-        const unsigned mm = ap.span_mul[f];
-        switch (R) {
-            case 2: stage<2, INV>(buf, ln, ap.n, m, mm, tw); break;
-            case 3: stage<3, INV>(buf, ln, ap.n, m, mm, tw); break;
-            case 4: stage<4, INV>(buf, ln, ap.n, m, mm, tw); break;
-            case 5: stage<5, INV>(buf, ln, ap.n, m, mm, tw); break;
-            case 6: stage<6, INV>(buf, ln, ap.n, m, mm, tw); break;
-            case 7: stage<7, INV>(buf, ln, ap.n, m, mm, tw); break;
-            case 8: stage<8, INV>(buf, ln, ap.n, m, mm, tw); break;
-            case 9: stage<9, INV>(buf, ln, ap.n, m, mm, tw); break;
-            case 10: stage<10, INV>(buf, ln, ap.n, m, mm, tw); break;
-            case 11: stage<11, INV>(buf, ln, ap.n, m, mm, tw); break;
-            case 12: stage<12, INV>(buf, ln, ap.n, m, mm, tw); break;
-            case 13: stage<13, INV>(buf, ln, ap.n, m, mm, tw); break;
-            case 16: stage<16, INV>(buf, ln, ap.n, m, mm, tw); break;
-            default: stage_prime<INV>(buf, ln, R, ap.n, m, mm, tw); break;
-        }
-        if (!INV) m *= R;
-        __syncthreads();
-    }
+__device__ __forceinline__ void transform(C *buf, const Lines ln, const Axis &ap, const C *tw) {
+    for (int i = 0; i < ap.nf; i++) run_stage<INV>(buf, ln, ap.st[INV ? i : ap.nf - 1 - i], tw);
 }
 
 }  // namespace any

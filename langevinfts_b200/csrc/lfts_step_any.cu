@@ -68,10 +68,9 @@ bool make_axis(int n, any::Axis &ax, std::vector<short> &perm, std::vector<short
     ax.n = n;
     ax.nf = (int)r.size();
     int span = n;
-    for (int f = 0; f < any::MAXF; f++) {
-        ax.radix[f] = f < ax.nf ? r[f] : 1;
-        if (f < ax.nf) span /= r[f];
-        ax.span_mul[f] = any::div_mul(f < ax.nf ? span : 1);
+    for (int f = 0; f < ax.nf; f++) {
+        span /= r[f];
+        ax.st[f] = {r[f], span, any::div_mul(span), n / r[f], n / (span * r[f])};
     }
     perm.assign(n, 0);
     iperm.assign(n, 0);
@@ -99,21 +98,30 @@ template <typename T> bool allow_all(int max_smem) {
     return allow(any::ka_plane_forward<T, true>, max_smem) && allow(any::ka_plane_forward<T, false>, max_smem) &&
            allow(any::ka_plane_mid<T>, max_smem) && allow(any::ka_plane_inverse<T, true>, max_smem) &&
            allow(any::ka_plane_inverse<T, false>, max_smem) && allow(any::ka_xpass<T, 1>, max_smem) &&
-           allow(any::ka_xpass<T, 2>, max_smem) && allow(any::ka_xpass_forward<T>, max_smem) &&
+           allow(any::ka_xpass<T, 2>, max_smem) && allow(any::ka_xpass_forward<T>, max_smem) && allow(any::ka_xstress<T>, max_smem) &&
            allow(any::ka_sweep_continuous<T>, max_smem, true) && allow(any::ka_sweep_discrete<T>, max_smem, true);
 }
 
 int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+any::Stack stack(const Plan &g, int planes) { return {planes, any::div_mul(planes * g.n1), any::div_mul(planes * g.n2)}; }
+
 struct SweepShape {
-    int XB, JB;
+    any::Sweep w;
     size_t smem;
 };
 template <typename C> SweepShape sweep_shape(const Plan &g, bool continuous, int cs) {
     SweepShape s;
-    s.XB = ceil_div(g.n0, cs);
-    s.JB = ceil_div(g.n1 * g.nzc, cs);
-    s.smem = continuous ? any::SweepBuf<C>::bytes(g, s.XB, 2 * s.JB) : any::SweepBuf<C>::bytes(g, (s.XB + 1) / 2, s.JB);
+    any::Sweep &w = s.w;
+    w.XB = ceil_div(g.n0, cs);
+    w.JB = ceil_div(g.n1 * g.nzc, cs);
+    w.width = continuous ? 2 * w.JB : w.JB;
+    w.mul_xb = any::div_mul(w.XB);
+    w.mul_jb = any::div_mul(w.JB);
+    w.mul_width = any::div_mul(w.width);
+    w.all = stack(g, w.XB);
+    w.half = stack(g, (w.XB + 1) / 2);
+    s.smem = any::SweepBuf<C>::bytes(g, continuous ? w.XB : w.half.planes, w.width);
     return s;
 }
 SweepShape sweep_shape(const AnyGrid *a, bool continuous, int cs) {
@@ -121,7 +129,7 @@ SweepShape sweep_shape(const AnyGrid *a, bool continuous, int cs) {
 }
 int sweep_threads(const AnyGrid *a, const SweepShape &s) {
     // a thread for every four points of the slab's packed planes
-    const int want = s.XB * a->p.n1 * a->p.n2 / 4;
+    const int want = s.w.XB * a->p.n1 * a->p.n2 / 4;
     return std::min(any::NT_MAX, std::max(128, (want + 31) / 32 * 32));
 }
 
@@ -215,7 +223,7 @@ template <typename C> int tile_columns(const AnyGrid *a, int nbr, int nj) {
     const int cols = g.n1 * g.nzc;
     // narrower tiles (still whole 64-byte rows) when wide ones leave SMs without work or do not fit
     while (tj > 4 && (any::TileBuf<C>::bytes(g, nbr * tj) > (size_t)a->max_smem ||
-                      ((long long)ceil_div(cols, tj) * nj < a->nsm && tj * sizeof(C) > 64)))
+                      ((long long)ceil_div(cols, tj) * nj < a->nsm && tj * sizeof(C) > 128)))
         tj /= 2;
     return tj;
 }
@@ -225,21 +233,21 @@ template <typename T, bool TWO> void plane_forward(const AnyGrid *a, cudaStream_
     const Plan &g = a->p;
     const int units = TWO ? g.n0 : ceil_div(g.n0, 2), k = stack_planes<C>(a, units, nj), ctas = ceil_div(units, k);
     any::ka_plane_forward<T, TWO><<<dim3(ctas, nj), plane_threads(a, ctas * nj, k * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, k), st>>>(
-        g, jobs, s, f0, f1, spec, k);
+        g, jobs, s, f0, f1, spec, stack(g, k));
 }
 template <typename T, bool TWO> void plane_inverse(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s, int spec, int f0) {
     using C = typename CT<T>::type;
     const Plan &g = a->p;
     const int units = TWO ? g.n0 : ceil_div(g.n0, 2), k = stack_planes<C>(a, units, nj), ctas = ceil_div(units, k);
     any::ka_plane_inverse<T, TWO><<<dim3(ctas, nj), plane_threads(a, ctas * nj, k * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, k), st>>>(
-        g, jobs, s, spec, f0, k);
+        g, jobs, s, spec, f0, stack(g, k));
 }
 template <typename T, int NBR> void xpass(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int spec, int b0, int b1) {
     using C = typename CT<T>::type;
     const Plan &g = a->p;
     const int tj = tile_columns<C>(a, NBR, nj), ctas = ceil_div(g.n1 * g.nzc, tj);
     any::ka_xpass<T, NBR><<<dim3(ctas, nj), plane_threads(a, ctas * nj, g.n0 * tj * NBR), any::TileBuf<C>::bytes(g, NBR * tj), st>>>(
-        g, jobs, spec, b0, b1, tj, any::div_mul(tj));
+        g, jobs, spec, b0, b1, tj, any::div_mul(tj), any::div_mul(NBR * tj));
 }
 template <typename T> void step_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s) {
     using C = typename CT<T>::type;
@@ -247,7 +255,7 @@ template <typename T> void step_continuous(const AnyGrid *a, cudaStream_t st, co
     plane_forward<T, true>(a, st, jobs, nj, s, FM_FAC_SQ, FM_FAC, 0);
     xpass<T, 2>(a, st, jobs, nj, 0, 0, 1);
     const int units = ceil_div(g.n0, 2), k = stack_planes<C>(a, units, nj), ctas = ceil_div(units, k);
-    any::ka_plane_mid<T><<<dim3(ctas, nj), plane_threads(a, ctas * nj, k * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, k), st>>>(g, jobs, 1, k);
+    any::ka_plane_mid<T><<<dim3(ctas, nj), plane_threads(a, ctas * nj, k * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, k), st>>>(g, jobs, 1, stack(g, k));
     xpass<T, 1>(a, st, jobs, nj, 1, 1, 1);
     plane_inverse<T, true>(a, st, jobs, nj, s, 0, 0);
 }
@@ -261,22 +269,29 @@ template <typename T> void xforward(const AnyGrid *a, cudaStream_t st, const lft
     const Plan &g = a->p;
     const int tj = tile_columns<C>(a, 1, nj), ctas = ceil_div(g.n1 * g.nzc, tj);
     any::ka_xpass_forward<T><<<dim3(ctas, nj), plane_threads(a, ctas * nj, g.n0 * tj), any::TileBuf<C>::bytes(g, tj), st>>>(
-        g, jobs, tj, any::div_mul(tj));
+        g, jobs, tj, any::div_mul(tj), any::div_mul(tj));
+}
+template <typename T> void xstress(const AnyGrid *a, cudaStream_t st, const lfts_step_job *sj, const lfts_stress_job *jobs, int nj,
+                                   const double *basis, double *partials) {
+    using C = typename CT<T>::type;
+    const Plan &g = a->p;
+    const int tj = tile_columns<C>(a, 2, nj);
+    any::ka_xstress<T><<<dim3(ceil_div(g.n1 * g.nzc, tj), nj), NTHR, any::TileBuf<C>::bytes(g, 2 * tj), st>>>(
+        g, sj, jobs, basis, tj, any::div_mul(tj), any::div_mul(2 * tj), partials);
 }
 template <typename T> int sweep_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int n, int cs) {
     const SweepShape s = sweep_shape(a, true, cs);
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at;
     cluster_config(cfg, &at, any::ka_sweep_continuous<T>, cs, nj, sweep_threads(a, s), s.smem, st);
-    return (int)cudaLaunchKernelEx(&cfg, any::ka_sweep_continuous<T>, a->p, jobs, s0, n, s.XB, any::div_mul(s.XB), s.JB, any::div_mul(s.JB));
+    return (int)cudaLaunchKernelEx(&cfg, any::ka_sweep_continuous<T>, a->p, s.w, jobs, s0, n);
 }
 template <typename T> int sweep_discrete(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int n, int half, int wf, int cs) {
     const SweepShape s = sweep_shape(a, false, cs);
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at;
     cluster_config(cfg, &at, any::ka_sweep_discrete<T>, cs, nj, sweep_threads(a, s), s.smem, st);
-    return (int)cudaLaunchKernelEx(&cfg, any::ka_sweep_discrete<T>, a->p, jobs, s0, n, half, wf, s.XB, any::div_mul(s.XB), s.JB,
-                                   any::div_mul(s.JB));
+    return (int)cudaLaunchKernelEx(&cfg, any::ka_sweep_discrete<T>, a->p, s.w, jobs, s0, n, half, wf);
 }
 }  // namespace
 
@@ -321,6 +336,19 @@ void any_planes_forward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *
 void any_xpass_forward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj) {
     a->prec == 8 ? xforward<double>(a, st, jobs, nj) : xforward<float>(a, st, jobs, nj);
 }
+int any_stress_tiles(const AnyGrid *a, int nj) {
+    return ceil_div(a->p.n1 * a->p.nzc, a->prec == 8 ? tile_columns<double2>(a, 2, nj) : tile_columns<float2>(a, 2, nj));
+}
+void any_xstress(const AnyGrid *a, cudaStream_t st, const lfts_step_job *sj, const lfts_stress_job *jobs, int nj, const double *basis,
+                 double *partials) {
+    a->prec == 8 ? xstress<double>(a, st, sj, jobs, nj, basis, partials) : xstress<float>(a, st, sj, jobs, nj, basis, partials);
+}
+// A sweep's step costs barriers and transposes whatever the grid, then time per point
+// a CTA holds; the separate passes cost five (discrete: three) launches, then time per
+// point of all jobs.  Microseconds measured on a B200, FP64 (FP32): 84 x 48, 2 jobs 20.3 a
+// step in clusters of 16 against 27.7 (17.7 / 27.9); 256 points 16.2 / 25.4; 24^3 25 / 30;
+// 32^3, 32 768 points, 32.5 / 32.0 (26.6 / 30.4): the lines cross near 1500 (2500) points a
+// CTA.  More clusters than the device holds at once run in waves.
 int any_sweep_size(const AnyGrid *a, bool continuous, int nj, int force) {
     const int *res = continuous ? a->clusters_cont : a->clusters_disc;
     if (force) {
@@ -328,7 +356,20 @@ int any_sweep_size(const AnyGrid *a, bool continuous, int nj, int force) {
             if (1 << k == force && res[k]) return force;
         return 0;
     }
-    return 0;
+    const bool f64 = a->prec == 8;
+    const double M = (double)a->p.M, part = continuous ? 1.0 : 0.55;
+    const double fixed = f64 ? 17.5 : 14.5, per_point = f64 ? 7.3e-3 : 4.8e-3;
+    double best = part * (26.0 + nj * M * (f64 ? 5e-5 : 4e-5));
+    int size = 0;
+    for (int k = 0; k < 5; k++) {
+        if (!res[k]) continue;
+        const double t = part * ((nj + res[k] - 1) / res[k]) * (fixed + per_point * M / (1 << k));
+        if (t < best) {
+            best = t;
+            size = 1 << k;
+        }
+    }
+    return size;
 }
 int any_sweep_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps, int cs) {
     return a->prec == 8 ? sweep_continuous<double>(a, st, jobs, nj, s0, nsteps, cs) : sweep_continuous<float>(a, st, jobs, nj, s0, nsteps, cs);

@@ -15,7 +15,7 @@
 // memory.  q is written once a step and nothing else reaches HBM.
 #pragma once
 #include "lfts_fft_any.cuh"
-#include "lfts_step_kernels.cuh"
+#include "lfts_reduce.cuh"
 
 namespace lfts {
 namespace any {
@@ -40,24 +40,28 @@ struct PlaneBuf {
     }
 };
 
-// z lines (rows) and y lines (columns) of `planes` stacked planes
-__device__ __forceinline__ Lines z_lines(const Plan &g, int planes) {
-    const int nl = planes * g.n1;
-    return {nl, div_mul(nl), g.pitch, 1, 0u, 0};
+// Packed planes stacked in one buffer, with the divisions of their line counts
+// (prepared by the host; a CTA with fewer planes transforms the unused ones too)
+struct Stack {
+    int planes;
+    unsigned mul_rows, mul_cols;  // division by planes * n1 and by planes * n2
+};
+// z lines (rows) and y lines (columns)
+__device__ __forceinline__ Lines z_lines(const Plan &g, const Stack &k) {
+    return {k.planes * g.n1, k.mul_rows, g.pitch, 1, 0u, 0};
 }
-__device__ __forceinline__ Lines y_lines(const Plan &g, int planes) {
-    const int nl = planes * g.n2;
-    return {nl, div_mul(nl), 1, g.pitch, g.mul_n2, planes > 1 ? g.n1 * g.pitch - g.n2 : 0};
+__device__ __forceinline__ Lines y_lines(const Plan &g, const Stack &k) {
+    return {k.planes * g.n2, k.mul_cols, 1, g.pitch, g.mul_n2, k.planes > 1 ? g.n1 * g.pitch - g.n2 : 0};
 }
 template <typename C>
-__device__ __forceinline__ void plane_forward(const Plan &g, C *buf, int planes, const C *twy, const C *twz) {
-    transform<false>(buf, z_lines(g, planes), g.ax[2], twz);
-    transform<false>(buf, y_lines(g, planes), g.ax[1], twy);
+__device__ __forceinline__ void plane_forward(const Plan &g, C *buf, const Stack &k, const C *twy, const C *twz) {
+    transform<false>(buf, z_lines(g, k), g.ax[2], twz);
+    transform<false>(buf, y_lines(g, k), g.ax[1], twy);
 }
 template <typename C>
-__device__ __forceinline__ void plane_inverse(const Plan &g, C *buf, int planes, const C *twy, const C *twz) {
-    transform<true>(buf, y_lines(g, planes), g.ax[1], twy);
-    transform<true>(buf, z_lines(g, planes), g.ax[2], twz);
+__device__ __forceinline__ void plane_inverse(const Plan &g, C *buf, const Stack &k, const C *twy, const C *twz) {
+    transform<true>(buf, y_lines(g, k), g.ax[1], twy);
+    transform<true>(buf, z_lines(g, k), g.ax[2], twz);
 }
 
 // Half spectra of the two real planes a packed plane carries, at (ky, kz)
@@ -99,15 +103,15 @@ constexpr int U = 4;  // independent global loads a thread keeps in flight
 // Otherwise planes 2p, 2p + 1 with factor fm0 -> spectrum spec_out.
 template <typename T, bool TWO>
 __global__ void __launch_bounds__(NT_MAX) ka_plane_forward(const __grid_constant__ Plan g, const lfts_step_job *__restrict__ jobs, int s, int fm0,
-                                                           int fm1, int spec_out, int planes) {
+                                                           int fm1, int spec_out, Stack sk) {
     using C = typename CT<T>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    PlaneBuf<C> sm(smem_raw, g, planes);
+    PlaneBuf<C> sm(smem_raw, g, sk.planes);
     const lfts_step_job jb = jobs[blockIdx.y];
     if (jb.active && !jb.active[jb.replica]) return;
     __syncthreads();
-    const int per = TWO ? 1 : 2, x0 = blockIdx.x * planes * per;
-    const int nx = min(planes * per, g.n0 - x0), np = (nx + per - 1) / per, area = g.n1 * g.n2;
+    const int per = TWO ? 1 : 2, x0 = blockIdx.x * sk.planes * per;
+    const int nx = min(sk.planes * per, g.n0 - x0), np = (nx + per - 1) / per, area = g.n1 * g.n2;
     const T *qin = (const T *)jb.in + s * jb.in_stride + (long long)x0 * area;
     const T *fac = (const T *)jb.fac + (long long)x0 * area;
     const int tot = np * area;
@@ -147,7 +151,7 @@ __global__ void __launch_bounds__(NT_MAX) ka_plane_forward(const __grid_constant
         }
     }
     __syncthreads();
-    plane_forward(g, sm.buf, np, sm.twy, sm.twz);
+    plane_forward(g, sm.buf, sk, sm.twy, sm.twz);
     const int half = g.n1 * g.nzc;
     C *out = (C *)jb.spec + (size_t)(TWO ? 0 : spec_out) * g.Mc + (size_t)x0 * half;
     for (int i = threadIdx.x; i < np * half; i += blockDim.x) {
@@ -206,18 +210,18 @@ __device__ __forceinline__ void load_packed(const Plan &g, const C *__restrict__
 // ------------------------------------------------------------------------
 // K3: inverse zy of planes 2p, 2p + 1, multiply by fac^2, forward zy, in place
 template <typename T>
-__global__ void __launch_bounds__(NT_MAX) ka_plane_mid(const __grid_constant__ Plan g, const lfts_step_job *__restrict__ jobs, int spec_idx, int planes) {
+__global__ void __launch_bounds__(NT_MAX) ka_plane_mid(const __grid_constant__ Plan g, const lfts_step_job *__restrict__ jobs, int spec_idx, Stack sk) {
     using C = typename CT<T>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    PlaneBuf<C> sm(smem_raw, g, planes);
+    PlaneBuf<C> sm(smem_raw, g, sk.planes);
     const lfts_step_job jb = jobs[blockIdx.y];
     if (jb.active && !jb.active[jb.replica]) return;
-    const int x0 = blockIdx.x * planes * 2, nx = min(planes * 2, g.n0 - x0), np = (nx + 1) / 2;
+    const int x0 = blockIdx.x * sk.planes * 2, nx = min(sk.planes * 2, g.n0 - x0), np = (nx + 1) / 2;
     const int area = g.n1 * g.n2, half = g.n1 * g.nzc;
     C *spec = (C *)jb.spec + (size_t)spec_idx * g.Mc + (size_t)x0 * half;
     load_packed<C, false>(g, spec, sm.buf, np, nx);
     __syncthreads();
-    plane_inverse(g, sm.buf, np, sm.twy, sm.twz);
+    plane_inverse(g, sm.buf, sk, sm.twy, sm.twz);
     const T *fac = (const T *)jb.fac + (long long)x0 * area;
     for (int i = threadIdx.x; i < np * area; i += blockDim.x) {
         const Point pt = point_at(g, i, sm.iy, sm.iz);
@@ -229,7 +233,7 @@ __global__ void __launch_bounds__(NT_MAX) ka_plane_mid(const __grid_constant__ P
         sm.buf[pt.o] = z;
     }
     __syncthreads();
-    plane_forward(g, sm.buf, np, sm.twy, sm.twz);
+    plane_forward(g, sm.buf, sk, sm.twy, sm.twz);
     for (int i = threadIdx.x; i < np * half; i += blockDim.x) {
         const int r = fdiv(i, g.mul_nzc), kz = i - r * g.nzc;
         const int p = fdiv(r, g.mul_n1), ky = r - p * g.n1;
@@ -246,17 +250,17 @@ __global__ void __launch_bounds__(NT_MAX) ka_plane_mid(const __grid_constant__ P
 // q' = v * factor(fm0) of planes 2p, 2p + 1.
 template <typename T, bool TWO>
 __global__ void __launch_bounds__(NT_MAX) ka_plane_inverse(const __grid_constant__ Plan g, const lfts_step_job *__restrict__ jobs, int s, int spec_in,
-                                                           int fm0, int planes) {
+                                                           int fm0, Stack sk) {
     using C = typename CT<T>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    PlaneBuf<C> sm(smem_raw, g, planes);
+    PlaneBuf<C> sm(smem_raw, g, sk.planes);
     const lfts_step_job jb = jobs[blockIdx.y];
     if (jb.active && !jb.active[jb.replica]) return;
-    const int per = TWO ? 1 : 2, x0 = blockIdx.x * planes * per;
-    const int nx = min(planes * per, g.n0 - x0), np = (nx + per - 1) / per, area = g.n1 * g.n2, half = g.n1 * g.nzc;
+    const int per = TWO ? 1 : 2, x0 = blockIdx.x * sk.planes * per;
+    const int nx = min(sk.planes * per, g.n0 - x0), np = (nx + per - 1) / per, area = g.n1 * g.n2, half = g.n1 * g.nzc;
     load_packed<C, TWO>(g, (const C *)jb.spec + (size_t)(TWO ? 0 : spec_in) * g.Mc + (size_t)x0 * half, sm.buf, np, nx);
     __syncthreads();
-    plane_inverse(g, sm.buf, np, sm.twy, sm.twz);
+    plane_inverse(g, sm.buf, sk, sm.twy, sm.twz);
     const T *fac = (const T *)jb.fac + (long long)x0 * area;
     T *qout = (T *)jb.out + s * jb.out_stride + (long long)x0 * area;
     for (int i = threadIdx.x; i < np * area; i += blockDim.x) {
@@ -323,7 +327,7 @@ __device__ __forceinline__ void load_tile(const Plan &g, const C *__restrict__ s
 // K2 / K4: x-transform, bond tables, inverse
 template <typename T, int NBR>
 __global__ void __launch_bounds__(NT_MAX) ka_xpass(const __grid_constant__ Plan g, const lfts_step_job *__restrict__ jobs, int spec_in, int bsel0,
-                                                   int bsel1, int TJ, unsigned mul_tj) {
+                                                   int bsel1, int TJ, unsigned mul_tj, unsigned mul_w) {
     using C = typename CT<T>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TileBuf<C> sm(smem_raw, g, NBR * TJ);
@@ -334,7 +338,7 @@ __global__ void __launch_bounds__(NT_MAX) ka_xpass(const __grid_constant__ Plan 
     C *spec = (C *)jb.spec + (size_t)spec_in * g.Mc;
     load_tile<C, NBR>(g, spec, sm, j0, nj, TJ, mul_tj);
     __syncthreads();
-    const Lines lx = {NBR * TJ, div_mul(NBR * TJ), 1, NBR * TJ, 0u, 0};
+    const Lines lx = {NBR * TJ, mul_w, 1, NBR * TJ, 0u, 0};
     transform<false>(sm.tile, lx, g.ax[0], sm.twx);
     const T *bt0 = (const T *)(bsel0 ? jb.bond_half : jb.bond), *bt1 = (const T *)(bsel1 ? jb.bond_half : jb.bond);
     for (int i = threadIdx.x; i < g.n0 * TJ; i += blockDim.x) {
@@ -366,7 +370,7 @@ __global__ void __launch_bounds__(NT_MAX) ka_xpass(const __grid_constant__ Plan 
 
 // Forward x-transform only: completes a 3D real transform
 template <typename T>
-__global__ void __launch_bounds__(NT_MAX) ka_xpass_forward(const __grid_constant__ Plan g, const lfts_step_job *__restrict__ jobs, int TJ, unsigned mul_tj) {
+__global__ void __launch_bounds__(NT_MAX) ka_xpass_forward(const __grid_constant__ Plan g, const lfts_step_job *__restrict__ jobs, int TJ, unsigned mul_tj, unsigned mul_w) {
     using C = typename CT<T>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TileBuf<C> sm(smem_raw, g, TJ);
@@ -377,11 +381,49 @@ __global__ void __launch_bounds__(NT_MAX) ka_xpass_forward(const __grid_constant
     C *spec = (C *)jb.spec;
     load_tile<C, 1>(g, spec, sm, j0, nj, TJ, mul_tj);
     __syncthreads();
-    const Lines lx = {TJ, div_mul(TJ), 1, TJ, 0u, 0};
+    const Lines lx = {TJ, mul_w, 1, TJ, 0u, 0};
     transform<false>(sm.tile, lx, g.ax[0], sm.twx);
     for (int i = threadIdx.x; i < g.n0 * TJ; i += blockDim.x) {
         const int x = fdiv(i, mul_tj), jj = i - x * TJ;
         if (jj < nj) spec[(long long)x * plane + j0 + jj] = sm.tile[x * TJ + jj];
+    }
+}
+
+// Stress of one (q1, q2) pair per job: x-transform of both zy spectra, then
+// sum_k Re(q1 q2*) basis_d(k).  Blocks of NTHR threads (the reductions' size).
+template <typename T>
+__global__ void __launch_bounds__(NTHR) ka_xstress(const __grid_constant__ Plan g, const lfts_step_job *__restrict__ sj,
+                                                   const lfts_stress_job *__restrict__ jobs, const double *__restrict__ basis,
+                                                   int TJ, unsigned mul_tj, unsigned mul_w, double *partials) {
+    using C = typename CT<T>::type;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double sh[2 * NWARP];
+    TileBuf<C> sm(smem_raw, g, 2 * TJ);
+    const int job = blockIdx.y;
+    const C *spec = (const C *)sj[2 * job].spec;  // two consecutive Mc slots
+    const T *bond = (const T *)jobs[job].bond;
+    __syncthreads();
+    const int plane = g.n1 * g.nzc, j0 = blockIdx.x * TJ, nj = min(TJ, plane - j0);
+    load_tile<C, 2>(g, spec, sm, j0, nj, TJ, mul_tj);
+    __syncthreads();
+    const Lines lx = {2 * TJ, mul_w, 1, 2 * TJ, 0u, 0};
+    transform<false>(sm.tile, lx, g.ax[0], sm.twx);
+    Acc<T> acc[3];
+    for (int i = threadIdx.x; i < g.n0 * TJ; i += blockDim.x) {
+        const int x = fdiv(i, mul_tj), jj = i - x * TJ;
+        if (jj < nj) {
+            const long long k = (long long)x * plane + j0 + jj;
+            const C A = sm.tile[x * (2 * TJ) + jj], B = sm.tile[x * (2 * TJ) + TJ + jj];
+            double co = (double)A.x * (double)B.x + (double)A.y * (double)B.y;
+            if (bond) co *= (double)bond[k] * (double)g.M;  // tables carry 1/M
+            acc[0].add(co * basis[k]);
+            acc[1].add(co * basis[g.Mc + k]);
+            acc[2].add(co * basis[2 * g.Mc + k]);
+        }
+    }
+    for (int d = 0; d < 3; d++) {
+        const double v = acc[d].block(sh);
+        if (threadIdx.x == 0) partials[((long long)job * gridDim.x + blockIdx.x) * 3 + d] = v;
     }
 }
 
@@ -437,44 +479,48 @@ struct SweepBuf {
     }
 };
 
+// The shape of a sweep, its divisions prepared by the host
+struct Sweep {
+    int XB, JB, width;   // planes and columns a CTA, columns side by side in col
+    unsigned mul_xb, mul_jb, mul_width;
+    Stack all, half;     // every plane packed by itself; planes packed in pairs
+};
+
 // slab -> columns.  PER = 1: every plane is packed by itself and gives the columns of
 // both branches (b at jj, b' at JB + jj); PER = 2: planes 2p, 2p + 1 packed, one branch
 // at column offset coff.
 template <typename C, int PER>
-__device__ __forceinline__ void pull_columns(const Plan &g, const SweepBuf<C> &sm, int XB, unsigned mul_xb, int j0, int nj,
-                                             int width, int JB, int coff) {
-    const unsigned mul_nj = div_mul(nj);
-    const int tot = g.n0 * nj;
+__device__ __forceinline__ void pull_columns(const Plan &g, const SweepBuf<C> &sm, const Sweep &w, int j0, int nj, int coff) {
+    const int tot = g.n0 * w.JB;
     const C zero = cmk<C>(0, 0);
     for (int i0 = threadIdx.x; i0 < tot; i0 += U * blockDim.x) {
         C z[U], zn[U];
+        int d[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int i = i0 + u * blockDim.x;
-            if (i < tot) {
-                const int x = fdiv(i, mul_nj), j = j0 + i - x * nj;
-                const int ky = fdiv(j, g.mul_nzc), kz = j - ky * g.nzc;
-                const int r = fdiv(x, mul_xb), p = (x - r * XB) / PER;
-                const int o = (p * g.n1 + ky) * g.pitch + kz;
-                const int on = (p * g.n1 + (ky ? g.n1 - ky : 0)) * g.pitch + (kz ? g.n2 - kz : 0);
-                z[u] = ld_remote(remote(sm.pl + o, r), zero);
-                zn[u] = ld_remote(remote(sm.pl + on, r), zero);
+            const int x = fdiv(i, w.mul_jb), jj = i - x * w.JB;
+            d[u] = -1;
+            if (i < tot && jj < nj) {
+                const int j = j0 + jj, ky = fdiv(j, g.mul_nzc), kz = j - ky * g.nzc;
+                const int r = fdiv(x, w.mul_xb), xl = x - r * w.XB;
+                const int row = (PER == 1 ? xl : xl >> 1) * g.n1;
+                z[u] = ld_remote(remote(sm.pl + (row + ky) * g.pitch + kz, r), zero);
+                zn[u] = ld_remote(remote(sm.pl + (row + (ky ? g.n1 - ky : 0)) * g.pitch + (kz ? g.n2 - kz : 0), r), zero);
+                d[u] = (sm.px[x] * w.width + jj) * 2 + (PER == 1 ? 0 : xl & 1);
             }
         }
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            const int i = i0 + u * blockDim.x;
-            if (i < tot) {
-                const int x = fdiv(i, mul_nj), jj = i - x * nj;
+            if (d[u] >= 0) {
                 C A, B;
                 separate(z[u], zn[u], A, B);
-                C *d = sm.col + sm.px[x] * width + jj;
+                C *o = sm.col + (d[u] >> 1);
                 if (PER == 1) {
-                    d[0] = A;
-                    d[JB] = B;
+                    o[0] = A;
+                    o[w.JB] = B;
                 } else {
-                    const int r = fdiv(x, mul_xb);
-                    d[coff] = (x - r * XB) & 1 ? B : A;
+                    o[coff] = d[u] & 1 ? B : A;
                 }
             }
         }
@@ -482,70 +528,82 @@ __device__ __forceinline__ void pull_columns(const Plan &g, const SweepBuf<C> &s
 }
 // columns -> packed planes of the slab (nx planes from x0), natural positions
 template <typename C, int PER>
-__device__ __forceinline__ void pull_planes(const Plan &g, const SweepBuf<C> &sm, int x0, int nx, int width, int JB,
-                                            unsigned mul_jb, int coff) {
-    const int half = g.n1 * g.nzc, np = (nx + PER - 1) / PER, tot = np * half;
+__device__ __forceinline__ void pull_planes(const Plan &g, const SweepBuf<C> &sm, const Sweep &w, int x0, int nx, int coff) {
+    const int half = g.n1 * g.nzc, tot = (nx + PER - 1) / PER * half;
     const C zero = cmk<C>(0, 0);
     for (int i0 = threadIdx.x; i0 < tot; i0 += U * blockDim.x) {
         C A[U], B[U];
+        int d[U], dn[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int i = i0 + u * blockDim.x;
             A[u] = B[u] = zero;
+            d[u] = dn[u] = -1;
             if (i < tot) {
-                const int rw = fdiv(i, g.mul_nzc), p = fdiv(rw, g.mul_n1), j = i - p * half;
-                const int r = fdiv(j, mul_jb), jj = j - r * JB;
+                const int rw = fdiv(i, g.mul_nzc), kz = i - rw * g.nzc;
+                const int p = fdiv(rw, g.mul_n1), ky = rw - p * g.n1, j = i - p * half;
+                const int r = fdiv(j, w.mul_jb), jj = j - r * w.JB;
                 const int x = x0 + p * PER;
-                const unsigned a = remote(sm.col + sm.px[x] * width + coff + jj, r);
+                const auto a = remote(sm.col + sm.px[x] * w.width + coff + jj, r);
                 A[u] = ld_remote(a, zero);
-                if (PER == 1) B[u] = ld_remote(a + JB * (unsigned)sizeof(C), zero);
-                else if (p * 2 + 1 < nx) B[u] = ld_remote(remote(sm.col + sm.px[x + 1] * width + coff + jj, r), zero);
+                if (PER == 1) B[u] = ld_remote(a + w.JB * (unsigned)sizeof(C), zero);
+                else if (p * 2 + 1 < nx) B[u] = ld_remote(remote(sm.col + sm.px[x + 1] * w.width + coff + jj, r), zero);
+                d[u] = rw * g.pitch + kz;
+                if (kz && 2 * kz != g.n2) dn[u] = (p * g.n1 + (ky ? g.n1 - ky : 0)) * g.pitch + g.n2 - kz;
             }
         }
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            const int i = i0 + u * blockDim.x;
-            if (i < tot) {
-                const int rw = fdiv(i, g.mul_nzc), kz = i - rw * g.nzc;
-                const int p = fdiv(rw, g.mul_n1), ky = rw - p * g.n1;
+            if (d[u] >= 0) {
                 C z, zn;
                 join(A[u], B[u], z, zn);
-                sm.pl[rw * g.pitch + kz] = z;
-                if (kz && 2 * kz != g.n2) sm.pl[(p * g.n1 + (ky ? g.n1 - ky : 0)) * g.pitch + g.n2 - kz] = zn;
+                sm.pl[d[u]] = z;
+                if (dn[u] >= 0) sm.pl[dn[u]] = zn;
             }
         }
     }
 }
-// x-transform of w columns from offset coff, bond multiply (mult), inverse
-template <typename C, typename T>
-__device__ __forceinline__ void columns_bond(const Plan &g, const SweepBuf<C> &sm, int j0, int nj, int width, int coff,
-                                             const T *__restrict__ bond) {
-    const unsigned mul_nj = div_mul(nj);
+// x-transform of the columns from coff, bond tables, inverse.  TWO: the columns of
+// both branches with their own tables.
+template <typename C, typename T, bool TWO>
+__device__ __forceinline__ void columns(const Plan &g, const SweepBuf<C> &sm, const Sweep &w, int j0, int nj, int coff,
+                                        const T *__restrict__ bond, const T *__restrict__ bond2) {
+    const Lines ln = {TWO ? w.width : w.JB, TWO ? w.mul_width : w.mul_jb, 1, w.width, 0u, 0};
+    transform<false>(sm.col + coff, ln, g.ax[0], sm.twx);
     const int plane = g.n1 * g.nzc;
-    for (int i = threadIdx.x; i < g.n0 * nj; i += blockDim.x) {
-        const int x = fdiv(i, mul_nj), jj = i - x * nj;
-        const T b = bond[x * plane + j0 + jj];
-        C *d = sm.col + x * width + coff + jj;
-        d->x *= b;
-        d->y *= b;
+    for (int i = threadIdx.x; i < g.n0 * w.JB; i += blockDim.x) {
+        const int x = fdiv(i, w.mul_jb), jj = i - x * w.JB;
+        if (jj < nj) {
+            const int k = x * plane + j0 + jj;
+            C *d = sm.col + x * w.width + coff + jj;
+            const T b = bond[k];
+            d->x *= b;
+            d->y *= b;
+            if (TWO) {
+                const T b2 = bond2[k];
+                d[w.JB].x *= b2;
+                d[w.JB].y *= b2;
+            }
+        }
     }
+    __syncthreads();
+    transform<true>(sm.col + coff, ln, g.ax[0], sm.twx);
 }
 
 // Continuous (Richardson) chains: steps s0 .. s0 + nsteps - 1 of every job.  Step
 // s + 1 starts from what step s wrote (out of s is in of s + 1).
 template <typename T>
-__global__ void __launch_bounds__(NT_MAX, 1) ka_sweep_continuous(const __grid_constant__ Plan g, const lfts_step_job *__restrict__ jobs, int s0, int nsteps,
-                                                                 int XB, unsigned mul_xb, int JB, unsigned mul_jb) {
+__global__ void __launch_bounds__(NT_MAX, 1) ka_sweep_continuous(const __grid_constant__ Plan g, const __grid_constant__ Sweep w,
+                                                                 const lfts_step_job *__restrict__ jobs, int s0, int nsteps) {
     using C = typename CT<T>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int width = 2 * JB;
-    SweepBuf<C> sm(smem_raw, g, XB, width);
+    SweepBuf<C> sm(smem_raw, g, w.XB, w.width);
     const lfts_step_job jb = jobs[blockIdx.y];
     if (jb.active && !jb.active[jb.replica]) return;  // the whole cluster: its CTAs share the job
     __syncthreads();
     const int rank = (int)cluster_rank(), area = g.n1 * g.n2;
-    const int x0 = rank * XB, nx = max(0, min(XB, g.n0 - x0)), np2 = (nx + 1) / 2;
-    const int j0 = rank * JB, nj = max(0, min(JB, g.n1 * g.nzc - j0));
+    const int x0 = rank * w.XB, nx = max(0, min(w.XB, g.n0 - x0)), np2 = (nx + 1) / 2;
+    const int j0 = rank * w.JB, nj = max(0, min(w.JB, g.n1 * g.nzc - j0));
     const T *fac = (const T *)jb.fac + (long long)x0 * area;
     const T *bond = (const T *)jb.bond, *bond_half = (const T *)jb.bond_half;
     const T *qin = (const T *)jb.in + s0 * jb.in_stride + (long long)x0 * area;
@@ -559,21 +617,16 @@ __global__ void __launch_bounds__(NT_MAX, 1) ka_sweep_continuous(const __grid_co
         sm.pl[pt.o] = z;
     }
     __syncthreads();
-    const Lines both = {width, div_mul(width), 1, width, 0u, 0}, second = {JB, div_mul(JB), 1, width, 0u, 0};
     for (int s = s0; s < s0 + nsteps; s++) {
-        plane_forward(g, sm.pl, nx, sm.twy, sm.twz);
+        plane_forward(g, sm.pl, w.all, sm.twy, sm.twz);
         cluster_sync();
-        pull_columns<C, 1>(g, sm, XB, mul_xb, j0, nj, width, JB, 0);
+        pull_columns<C, 1>(g, sm, w, j0, nj, 0);
         __syncthreads();
-        transform<false>(sm.col, both, g.ax[0], sm.twx);
-        columns_bond(g, sm, j0, nj, width, 0, bond);
-        columns_bond(g, sm, j0, nj, width, JB, bond_half);
-        __syncthreads();
-        transform<true>(sm.col, both, g.ax[0], sm.twx);
+        columns<C, T, true>(g, sm, w, j0, nj, 0, bond, bond_half);
         cluster_sync();
-        pull_planes<C, 2>(g, sm, x0, nx, width, JB, mul_jb, JB);  // the half-step branch only
+        pull_planes<C, 2>(g, sm, w, x0, nx, w.JB);  // the half-step branch only
         __syncthreads();
-        plane_inverse(g, sm.pl, np2, sm.twy, sm.twz);
+        plane_inverse(g, sm.pl, w.half, sm.twy, sm.twz);
         for (int i = threadIdx.x; i < np2 * area; i += blockDim.x) {
             const Point pt = point_at(g, i, sm.iy, sm.iz);
             const int src = (2 * pt.p * g.n1 + pt.y) * g.n2 + pt.t;
@@ -584,18 +637,15 @@ __global__ void __launch_bounds__(NT_MAX, 1) ka_sweep_continuous(const __grid_co
             sm.pl[pt.o] = z;
         }
         __syncthreads();
-        plane_forward(g, sm.pl, np2, sm.twy, sm.twz);
+        plane_forward(g, sm.pl, w.half, sm.twy, sm.twz);
         cluster_sync();
-        pull_columns<C, 2>(g, sm, XB, mul_xb, j0, nj, width, JB, JB);
+        pull_columns<C, 2>(g, sm, w, j0, nj, w.JB);
         __syncthreads();
-        transform<false>(sm.col + JB, second, g.ax[0], sm.twx);
-        columns_bond(g, sm, j0, nj, width, JB, bond_half);
-        __syncthreads();
-        transform<true>(sm.col + JB, second, g.ax[0], sm.twx);
+        columns<C, T, false>(g, sm, w, j0, nj, w.JB, bond_half, bond_half);
         cluster_sync();
-        pull_planes<C, 1>(g, sm, x0, nx, width, JB, mul_jb, 0);
+        pull_planes<C, 1>(g, sm, w, x0, nx, 0);
         __syncthreads();
-        plane_inverse(g, sm.pl, nx, sm.twy, sm.twz);
+        plane_inverse(g, sm.pl, w.all, sm.twy, sm.twz);
         T *qout = (T *)jb.out + s * jb.out_stride + (long long)x0 * area;
         for (int i = threadIdx.x; i < nx * area; i += blockDim.x) {
             const Point pt = point_at(g, i, sm.iy, sm.iz);
@@ -615,18 +665,18 @@ __global__ void __launch_bounds__(NT_MAX, 1) ka_sweep_continuous(const __grid_co
 
 // Discrete chains (and half-bond steps): q' = factor * conv(q, bond)
 template <typename T>
-__global__ void __launch_bounds__(NT_MAX, 1) ka_sweep_discrete(const __grid_constant__ Plan g, const lfts_step_job *__restrict__ jobs, int s0, int nsteps,
-                                                               int half_bond, int with_fac, int XB, unsigned mul_xb, int JB,
-                                                               unsigned mul_jb) {
+__global__ void __launch_bounds__(NT_MAX, 1) ka_sweep_discrete(const __grid_constant__ Plan g, const __grid_constant__ Sweep w,
+                                                               const lfts_step_job *__restrict__ jobs, int s0, int nsteps,
+                                                               int half_bond, int with_fac) {
     using C = typename CT<T>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    SweepBuf<C> sm(smem_raw, g, (XB + 1) / 2, JB);
+    SweepBuf<C> sm(smem_raw, g, w.half.planes, w.JB);
     const lfts_step_job jb = jobs[blockIdx.y];
     if (jb.active && !jb.active[jb.replica]) return;
     __syncthreads();
     const int rank = (int)cluster_rank(), area = g.n1 * g.n2;
-    const int x0 = rank * XB, nx = max(0, min(XB, g.n0 - x0)), np2 = (nx + 1) / 2;
-    const int j0 = rank * JB, nj = max(0, min(JB, g.n1 * g.nzc - j0));
+    const int x0 = rank * w.XB, nx = max(0, min(w.XB, g.n0 - x0)), np2 = (nx + 1) / 2;
+    const int j0 = rank * w.JB, nj = max(0, min(w.JB, g.n1 * g.nzc - j0));
     const T *fac = (const T *)jb.fac + (long long)x0 * area;
     const T *bond = (const T *)(half_bond ? jb.bond_half : jb.bond);
     const T *qin = (const T *)jb.in + s0 * jb.in_stride + (long long)x0 * area;
@@ -639,20 +689,16 @@ __global__ void __launch_bounds__(NT_MAX, 1) ka_sweep_discrete(const __grid_cons
         sm.pl[pt.o] = z;
     }
     __syncthreads();
-    const Lines lx = {JB, div_mul(JB), 1, JB, 0u, 0};
     for (int s = s0; s < s0 + nsteps; s++) {
-        plane_forward(g, sm.pl, np2, sm.twy, sm.twz);
+        plane_forward(g, sm.pl, w.half, sm.twy, sm.twz);
         cluster_sync();
-        pull_columns<C, 2>(g, sm, XB, mul_xb, j0, nj, JB, JB, 0);
+        pull_columns<C, 2>(g, sm, w, j0, nj, 0);
         __syncthreads();
-        transform<false>(sm.col, lx, g.ax[0], sm.twx);
-        columns_bond(g, sm, j0, nj, JB, 0, bond);
-        __syncthreads();
-        transform<true>(sm.col, lx, g.ax[0], sm.twx);
+        columns<C, T, false>(g, sm, w, j0, nj, 0, bond, bond);
         cluster_sync();
-        pull_planes<C, 2>(g, sm, x0, nx, JB, JB, mul_jb, 0);
+        pull_planes<C, 2>(g, sm, w, x0, nx, 0);
         __syncthreads();
-        plane_inverse(g, sm.pl, np2, sm.twy, sm.twz);
+        plane_inverse(g, sm.pl, w.half, sm.twy, sm.twz);
         T *qout = (T *)jb.out + s * jb.out_stride + (long long)x0 * area;
         for (int i = threadIdx.x; i < np2 * area; i += blockDim.x) {
             const Point pt = point_at(g, i, sm.iy, sm.iz);
