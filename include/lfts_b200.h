@@ -474,6 +474,16 @@ int lfts_adamw_f32(void *stream, float *p, const float *g, float *m, float *v, l
  * autograd of the ReLU and of the bias sum in the U-Net's training. */
 int lfts_relu_grad_bf16(void *stream, const void *gy, const void *y, void *g, float *db, long long npos, int cpad, int co);
 
+/* Between the U-Net's convolutions (no counterpart in the reference); BF16 arrays
+ * channels-last, channels multiples of 8, 16-byte aligned, stream as above.
+ * pack_input: FP32 [B][cin][D][H][W] -> BF16 [B][D][H][W][cpad], padding zero.
+ * pool: mean over 2 x 2 x 2 of x [B][D][H][W][cpad], summed in FP32.
+ * upcat: y [B][D][H][W][ca + cb] = a [B][D/2][H/2][W/2][ca] repeated twice along
+ * every axis, then b [B][D][H][W][cb]. */
+int lfts_unet_pack_input(void *stream, const float *x, void *y, int B, int cin, int D, int H, int W, int cpad);
+int lfts_unet_pool_bf16(void *stream, const void *x, void *y, int B, int D, int H, int W, int cpad);
+int lfts_unet_upcat_bf16(void *stream, const void *a, const void *b, void *y, int B, int D, int H, int W, int ca, int cb);
+
 /* Adam field update of the SCFT driver (examples/scft/scft.py:42-54), on n
  * doubles: m = b1 m + (1-b1) d; v = b2 v + (1-b2) d^2;
  * w_new = w + lr (m / (1 - b1^count)) / (sqrt(v / (1 - b2^count)) + eps).

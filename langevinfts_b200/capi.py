@@ -116,6 +116,9 @@ _SIGS = {
     "lfts_conv3d_bf16": [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int,
                          C.c_int, C.c_int, C.c_int, C.c_int],
     "lfts_relu_grad_bf16": [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_longlong, C.c_int, C.c_int],
+    "lfts_unet_pack_input": [C.c_void_p, C.c_void_p, C.c_void_p] + [C.c_int] * 6,
+    "lfts_unet_pool_bf16": [C.c_void_p, C.c_void_p, C.c_void_p] + [C.c_int] * 5,
+    "lfts_unet_upcat_bf16": [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p] + [C.c_int] * 6,
     "lfts_adamw_f32": [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_longlong, C.c_double, C.c_double,
                        C.c_double, C.c_double, C.c_double, C.c_int],
     "lfts_conv3d_wgrad_bf16": [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int,

@@ -41,8 +41,8 @@ Pieces:
                     writes the predicted w_+ in place on the engine's stream;
                     inference on the tensor cores by default.
 
-Pooling, upsampling and concatenation are torch tensor operations between the
-convolutions.  Grids must have extents divisible by 4.
+In training, pooling, upsampling and concatenation are torch tensor operations
+between the convolutions.  Grids must have extents divisible by 4.
 """
 import time
 
@@ -262,7 +262,8 @@ class TcgenUNet:
     """Inference of a trained UNet3D with every convolution on the tensor cores
     (lfts_conv3d_bf16: tcgen05 implicit GEMM, BF16 operands, FP32 accumulate);
     activations channels-last BF16 with channels padded to multiples of 16,
-    pooling / upsampling / concatenation as torch glue."""
+    pooling and upsampling with concatenation by one kernel each
+    (lfts_unet_pool_bf16, lfts_unet_upcat_bf16)."""
 
     def __init__(self, net):
         b = net.e1[0].out_channels
@@ -280,14 +281,37 @@ class TcgenUNet:
         self.out = pack_conv(net.out, rng(b), pb)
         self.cout = net.out.out_channels
 
-    @staticmethod
-    def _pool(x):
-        B, D, H, W, C = x.shape
-        return x.float().reshape(B, D // 2, 2, H // 2, 2, W // 2, 2, C).mean((2, 4, 6)).to(torch.bfloat16).contiguous()
+    def _pack(self, x):
+        """[B, cin, D, H, W] -> channels-last BF16 with padded channels (lfts_unet_pack_input for FP32 input)."""
+        from langevinfts_b200.capi import check, lib
+        if x.dtype != torch.float32 or not x.is_cuda:
+            h = x.permute(0, 2, 3, 4, 1).to(torch.bfloat16)
+            return F.pad(h, (0, self.cin_pad - h.shape[-1])).contiguous()
+        x = x.contiguous()
+        B, cin, D, H, W = x.shape
+        y = torch.empty([B, D, H, W, self.cin_pad], dtype=torch.bfloat16, device=x.device)
+        check(lib().lfts_unet_pack_input(torch.cuda.current_stream().cuda_stream, x.data_ptr(), y.data_ptr(), B, cin, D, H, W,
+                                         self.cin_pad))
+        return y
 
     @staticmethod
-    def _up(x):
-        return x.repeat_interleave(2, 1).repeat_interleave(2, 2).repeat_interleave(2, 3).contiguous()
+    def _pool(x):
+        from langevinfts_b200.capi import check, lib
+        B, D, H, W, C = x.shape
+        y = torch.empty([B, D // 2, H // 2, W // 2, C], dtype=torch.bfloat16, device=x.device)
+        check(lib().lfts_unet_pool_bf16(torch.cuda.current_stream().cuda_stream, x.data_ptr(), y.data_ptr(), B, D, H, W, C))
+        return y
+
+    @staticmethod
+    def _upcat(a, b):
+        """a upsampled to b's extents, then b, along the channels."""
+        from langevinfts_b200.capi import check, lib
+        B, D, H, W, cb = b.shape
+        ca = a.shape[-1]
+        y = torch.empty([B, D, H, W, ca + cb], dtype=torch.bfloat16, device=b.device)
+        check(lib().lfts_unet_upcat_bf16(torch.cuda.current_stream().cuda_stream, a.data_ptr(), b.data_ptr(), y.data_ptr(), B, D, H, W,
+                                         ca, cb))
+        return y
 
     def _block(self, x, pair):
         return conv3d_tcgen05(conv3d_tcgen05(x, pair[0], True), pair[1], True)
@@ -295,13 +319,11 @@ class TcgenUNet:
     @torch.no_grad()
     def __call__(self, x):
         """x: [B, cin, D, H, W] float -> [B, cout, D, H, W] float32."""
-        h = x.permute(0, 2, 3, 4, 1).to(torch.bfloat16)
-        h = torch.nn.functional.pad(h, (0, self.cin_pad - h.shape[-1])).contiguous()
-        x1 = self._block(h, self.e1)
+        x1 = self._block(self._pack(x), self.e1)
         x2 = self._block(self._pool(x1), self.e2)
         x3 = self._block(self._pool(x2), self.e3)
-        y2 = self._block(torch.cat([self._up(x3), x2], -1).contiguous(), self.d2)
-        y1 = self._block(torch.cat([self._up(y2), x1], -1).contiguous(), self.d1)
+        y2 = self._block(self._upcat(x3, x2), self.d2)
+        y1 = self._block(self._upcat(y2, x1), self.d1)
         o = conv3d_tcgen05(y1, self.out, False)[..., :self.cout]
         return o.permute(0, 4, 1, 2, 3).float().contiguous()
 
