@@ -600,6 +600,8 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3d_wgrad_umma(const uint4 *_
     } else if (warp < 4) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int co = 32 * warp + (tid & 31);  // accumulator row of this thread
+        // four sums an atomic where dw starts on 16 bytes (cin is a multiple of 16, so its rows then do too)
+        const bool vec = ((uintptr_t)dw & 15) == 0;
         for (int j = 0; j < ntap; j++) {
             const int tap = taps == 27 ? 3 * g + j : 0;
             for (int c0 = 0; c0 < cin; c0 += 16) {
@@ -607,8 +609,15 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3d_wgrad_umma(const uint4 *_
                 tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(j * cin + c0), v);
                 if (co < cout) {
                     float *o = dw + ((long long)tap * cout + co) * cin + c0;
+                    if (vec) {
 #pragma unroll
-                    for (int i = 0; i < 16; i++) atomicAdd(o + i, __uint_as_float(v[i]));
+                        for (int i = 0; i < 16; i += 4)
+                            atomicAdd((float4 *)(o + i), make_float4(__uint_as_float(v[i]), __uint_as_float(v[i + 1]),
+                                                                     __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])));
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; i++) atomicAdd(o + i, __uint_as_float(v[i]));
+                    }
                 }
             }
         }
