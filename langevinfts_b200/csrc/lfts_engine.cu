@@ -624,11 +624,11 @@ static int step_cont_fast(lfts_ctx c, const lfts_step_job *jobs, int nj, int s) 
             const size_t ps = r8::plane_smem<C>();
             const long long it2 = (long long)nj * 2 * r8::xpipe_tiles<C>(), it1 = (long long)nj * r8::xpipe_tiles<C>(), cap = (long long)(c->xcap ? c->xcap : 3) * c->nsm;
             const dim3 px2((unsigned)(it2 < cap ? it2 : cap)), px1((unsigned)(it1 < cap ? it1 : cap));
-            r8::kr_plane_forward<T, 2, FM_FAC_SQ, FM_FAC><<<rp, NTHR, ps, st>>>(g, jobs, s, 0);
-            r8::kp_xpass<T, 2><<<px2, NTHR, r8::xpipe_smem<C>(), st>>>(g, jobs, nj, 0, 0, 1);
-            r8::kr_plane_mid<T><<<rp, NTHR, ps, st>>>(g, jobs, 1);
-            r8::kp_xpass<T, 1><<<px1, NTHR, r8::xpipe_smem<C>(), st>>>(g, jobs, nj, 1, 1, 1);
-            r8::kr_plane_inverse<T, 2, EPI_RICH><<<rp, NTHR, ps, st>>>(g, jobs, s, 0, 0);
+            CK(launch_after(r8::kr_plane_forward<T, 2, FM_FAC_SQ, FM_FAC>, dim3(rp), NTHR, ps, st, g, jobs, s, 0));
+            CK(launch_after(r8::kp_xpass<T, 2>, dim3(px2), NTHR, r8::xpipe_smem<C>(), st, g, jobs, nj, 0, 0, 1));
+            CK(launch_after(r8::kr_plane_mid<T>, dim3(rp), NTHR, ps, st, g, jobs, 1));
+            CK(launch_after(r8::kp_xpass<T, 1>, dim3(px1), NTHR, r8::xpipe_smem<C>(), st, g, jobs, nj, 1, 1, 1));
+            CK(launch_after(r8::kr_plane_inverse<T, 2, EPI_RICH>, dim3(rp), NTHR, ps, st, g, jobs, s, 0, 0));
             CKLAUNCH();
             return 0;
         }
@@ -638,20 +638,20 @@ static int step_cont_fast(lfts_ctx c, const lfts_step_job *jobs, int nj, int s) 
             const size_t p2 = r12::plane_smem<C>(N), p1 = r12::plane_smem<C>(N / 2), xs = r12::xpipe_smem<C>();
             const long long it2 = (long long)nj * 2 * r12::XTILES, it1 = (long long)nj * r12::XTILES;
             const long long cap = (long long)(c->xcap ? c->xcap : r12::minb_xpass<T>()) * c->nsm;
-            r12::kq_plane_forward<T, FM_FAC_SQ, FM_FAC><<<gp, r12::NT, p2, st>>>(g, jobs, s, 0);
-            r12::kq_xpass<T, 2><<<(unsigned)(it2 < cap ? it2 : cap), NTHR, xs, st>>>(g, jobs, nj, 0, 0, 1);
-            r12::kq_plane_mid<T><<<gp, r12::NT, p1, st>>>(g, jobs, 1);
-            r12::kq_xpass<T, 1><<<(unsigned)(it1 < cap ? it1 : cap), NTHR, xs, st>>>(g, jobs, nj, 1, 1, 1);
-            r12::kq_plane_inverse<T><<<gp, r12::NT, p2, st>>>(g, jobs, s, 0);
+            CK(launch_after(r12::kq_plane_forward<T, FM_FAC_SQ, FM_FAC>, dim3(gp), r12::NT, p2, st, g, jobs, s, 0));
+            CK(launch_after(r12::kq_xpass<T, 2>, dim3((unsigned)(it2 < cap ? it2 : cap)), NTHR, xs, st, g, jobs, nj, 0, 0, 1));
+            CK(launch_after(r12::kq_plane_mid<T>, dim3(gp), r12::NT, p1, st, g, jobs, 1));
+            CK(launch_after(r12::kq_xpass<T, 1>, dim3((unsigned)(it1 < cap ? it1 : cap)), NTHR, xs, st, g, jobs, nj, 1, 1, 1));
+            CK(launch_after(r12::kq_plane_inverse<T>, dim3(gp), r12::NT, p2, st, g, jobs, s, 0));
             CKLAUNCH();
             return 0;
         }
     }
-    fast::kf_plane_forward<T, 2, N, NT2><<<gp, NT2, f2, st>>>(g, jobs, s, FM_FAC_SQ, FM_FAC, 0);
-    fast::kf_xpass<T, 2, N><<<gx, NTHR, x2, st>>>(g, jobs, 0, 0, 1);
-    fast::kf_plane_mid<T, N><<<gp, NTHR, f1, st>>>(g, jobs, 1);
-    fast::kf_xpass<T, 1, N><<<gx, NTHR, x1, st>>>(g, jobs, 1, 1, 1);
-    fast::kf_plane_inverse<T, 2, EPI_RICH, N, NT2><<<gp, NT2, f2, st>>>(g, jobs, s, 0, 0);
+    CK(launch_after(fast::kf_plane_forward<T, 2, N, NT2>, dim3(gp), NT2, f2, st, g, jobs, s, FM_FAC_SQ, FM_FAC, 0));
+    CK(launch_after(fast::kf_xpass<T, 2, N>, dim3(gx), NTHR, x2, st, g, jobs, 0, 0, 1));
+    CK(launch_after(fast::kf_plane_mid<T, N>, dim3(gp), NTHR, f1, st, g, jobs, 1));
+    CK(launch_after(fast::kf_xpass<T, 1, N>, dim3(gx), NTHR, x1, st, g, jobs, 1, 1, 1));
+    CK(launch_after(fast::kf_plane_inverse<T, 2, EPI_RICH, N, NT2>, dim3(gp), NT2, f2, st, g, jobs, s, 0, 0));
     CKLAUNCH();
     return 0;
 }
@@ -668,17 +668,17 @@ static int step_disc_fast(lfts_ctx c, const lfts_step_job *jobs, int nj, int s, 
         if (c->r8) {
             const dim3 rp(N, nj);
             const size_t ps = r8::plane_smem<C>();
-            r8::kr_plane_forward<T, 1, FM_NONE, FM_NONE><<<rp, NTHR, ps, st>>>(g, jobs, s, 0);
+            CK(launch_after(r8::kr_plane_forward<T, 1, FM_NONE, FM_NONE>, dim3(rp), NTHR, ps, st, g, jobs, s, 0));
             const long long it1 = (long long)nj * r8::xpipe_tiles<C>(), cap = (long long)(c->xcap ? c->xcap : 3) * c->nsm;
-            r8::kp_xpass<T, 1><<<(unsigned)(it1 < cap ? it1 : cap), NTHR, r8::xpipe_smem<C>(), st>>>(g, jobs, nj, 0, half, half);
-            r8::kr_plane_inverse<T, 1, EPI_SCALE><<<rp, NTHR, ps, st>>>(g, jobs, s, 0, with_fac ? FM_FAC : FM_NONE);
+            CK(launch_after(r8::kp_xpass<T, 1>, dim3((unsigned)(it1 < cap ? it1 : cap)), NTHR, r8::xpipe_smem<C>(), st, g, jobs, nj, 0, half, half));
+            CK(launch_after(r8::kr_plane_inverse<T, 1, EPI_SCALE>, dim3(rp), NTHR, ps, st, g, jobs, s, 0, with_fac ? FM_FAC : FM_NONE));
             CKLAUNCH();
             return 0;
         }
     }
-    fast::kf_plane_forward<T, 1, N><<<gp, NTHR, f1, st>>>(g, jobs, s, FM_NONE, 0, 0);
-    fast::kf_xpass<T, 1, N><<<gx, NTHR, x1, st>>>(g, jobs, 0, half, half);
-    fast::kf_plane_inverse<T, 1, EPI_SCALE, N><<<gp, NTHR, f1, st>>>(g, jobs, s, 0, with_fac ? FM_FAC : FM_NONE);
+    CK(launch_after(fast::kf_plane_forward<T, 1, N>, dim3(gp), NTHR, f1, st, g, jobs, s, FM_NONE, 0, 0));
+    CK(launch_after(fast::kf_xpass<T, 1, N>, dim3(gx), NTHR, x1, st, g, jobs, 0, half, half));
+    CK(launch_after(fast::kf_plane_inverse<T, 1, EPI_SCALE, N>, dim3(gp), NTHR, f1, st, g, jobs, s, 0, with_fac ? FM_FAC : FM_NONE));
     CKLAUNCH();
     return 0;
 }

@@ -228,26 +228,28 @@ template <typename C> int tile_columns(const AnyGrid *a, int nbr, int nj) {
     return tj;
 }
 
-template <typename T, bool TWO> void plane_forward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s, int f0, int f1, int spec) {
+// in_step: the job array is older than the kernel before this one
+template <typename T, bool TWO> void plane_forward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s, int f0, int f1, int spec, bool in_step = true) {
     using C = typename CT<T>::type;
     const Plan &g = a->p;
     const int units = TWO ? g.n0 : ceil_div(g.n0, 2), k = stack_planes<C>(a, units, nj), ctas = ceil_div(units, k);
-    any::ka_plane_forward<T, TWO><<<dim3(ctas, nj), plane_threads(a, ctas * nj, k * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, k), st>>>(
-        g, jobs, s, f0, f1, spec, stack(g, k));
+    const dim3 grid(ctas, nj);
+    const int threads = plane_threads(a, ctas * nj, k * g.n1 * g.n2);
+    const size_t smem = any::PlaneBuf<C>::bytes(g, k);
+    if (in_step) launch_after(any::ka_plane_forward<T, TWO>, grid, threads, smem, st, g, jobs, s, f0, f1, spec, stack(g, k));
+    else any::ka_plane_forward<T, TWO><<<grid, threads, smem, st>>>(g, jobs, s, f0, f1, spec, stack(g, k));
 }
 template <typename T, bool TWO> void plane_inverse(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s, int spec, int f0) {
     using C = typename CT<T>::type;
     const Plan &g = a->p;
     const int units = TWO ? g.n0 : ceil_div(g.n0, 2), k = stack_planes<C>(a, units, nj), ctas = ceil_div(units, k);
-    any::ka_plane_inverse<T, TWO><<<dim3(ctas, nj), plane_threads(a, ctas * nj, k * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, k), st>>>(
-        g, jobs, s, spec, f0, stack(g, k));
+    launch_after(any::ka_plane_inverse<T, TWO>, dim3(ctas, nj), plane_threads(a, ctas * nj, k * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, k), st, g, jobs, s, spec, f0, stack(g, k));
 }
 template <typename T, int NBR> void xpass(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int spec, int b0, int b1) {
     using C = typename CT<T>::type;
     const Plan &g = a->p;
     const int tj = tile_columns<C>(a, NBR, nj), ctas = ceil_div(g.n1 * g.nzc, tj);
-    any::ka_xpass<T, NBR><<<dim3(ctas, nj), plane_threads(a, ctas * nj, g.n0 * tj * NBR), any::TileBuf<C>::bytes(g, NBR * tj), st>>>(
-        g, jobs, spec, b0, b1, tj, any::div_mul(tj), any::div_mul(NBR * tj));
+    launch_after(any::ka_xpass<T, NBR>, dim3(ctas, nj), plane_threads(a, ctas * nj, g.n0 * tj * NBR), any::TileBuf<C>::bytes(g, NBR * tj), st, g, jobs, spec, b0, b1, tj, any::div_mul(tj), any::div_mul(NBR * tj));
 }
 template <typename T> void step_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s) {
     using C = typename CT<T>::type;
@@ -255,7 +257,7 @@ template <typename T> void step_continuous(const AnyGrid *a, cudaStream_t st, co
     plane_forward<T, true>(a, st, jobs, nj, s, FM_FAC_SQ, FM_FAC, 0);
     xpass<T, 2>(a, st, jobs, nj, 0, 0, 1);
     const int units = ceil_div(g.n0, 2), k = stack_planes<C>(a, units, nj), ctas = ceil_div(units, k);
-    any::ka_plane_mid<T><<<dim3(ctas, nj), plane_threads(a, ctas * nj, k * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, k), st>>>(g, jobs, 1, stack(g, k));
+    launch_after(any::ka_plane_mid<T>, dim3(ctas, nj), plane_threads(a, ctas * nj, k * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, k), st, g, jobs, 1, stack(g, k));
     xpass<T, 1>(a, st, jobs, nj, 1, 1, 1);
     plane_inverse<T, true>(a, st, jobs, nj, s, 0, 0);
 }
@@ -331,7 +333,7 @@ void any_step_discrete(const AnyGrid *a, cudaStream_t st, const lfts_step_job *j
     a->prec == 8 ? step_discrete<double>(a, st, jobs, nj, s, half, wf) : step_discrete<float>(a, st, jobs, nj, s, half, wf);
 }
 void any_planes_forward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj) {
-    a->prec == 8 ? plane_forward<double, false>(a, st, jobs, nj, 0, FM_NONE, 0, 0) : plane_forward<float, false>(a, st, jobs, nj, 0, FM_NONE, 0, 0);
+    a->prec == 8 ? plane_forward<double, false>(a, st, jobs, nj, 0, FM_NONE, 0, 0, false) : plane_forward<float, false>(a, st, jobs, nj, 0, FM_NONE, 0, 0, false);
 }
 void any_xpass_forward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj) {
     a->prec == 8 ? xforward<double>(a, st, jobs, nj) : xforward<float>(a, st, jobs, nj);

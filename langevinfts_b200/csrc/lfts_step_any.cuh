@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(NT_MAX) ka_plane_forward(const __grid_constant
     using C = typename CT<T>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PlaneBuf<C> sm(smem_raw, g, sk.planes);
+    grid_wait();
     const lfts_step_job jb = jobs[blockIdx.y];
     if (jb.active && !jb.active[jb.replica]) return;
     __syncthreads();
@@ -215,6 +216,7 @@ __global__ void __launch_bounds__(NT_MAX) ka_plane_mid(const __grid_constant__ P
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PlaneBuf<C> sm(smem_raw, g, sk.planes);
     const lfts_step_job jb = jobs[blockIdx.y];
+    grid_wait();
     if (jb.active && !jb.active[jb.replica]) return;
     const int x0 = blockIdx.x * sk.planes * 2, nx = min(sk.planes * 2, g.n0 - x0), np = (nx + 1) / 2;
     const int area = g.n1 * g.n2, half = g.n1 * g.nzc;
@@ -255,6 +257,7 @@ __global__ void __launch_bounds__(NT_MAX) ka_plane_inverse(const __grid_constant
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PlaneBuf<C> sm(smem_raw, g, sk.planes);
     const lfts_step_job jb = jobs[blockIdx.y];
+    grid_wait();
     if (jb.active && !jb.active[jb.replica]) return;
     const int per = TWO ? 1 : 2, x0 = blockIdx.x * sk.planes * per;
     const int nx = min(sk.planes * per, g.n0 - x0), np = (nx + per - 1) / per, area = g.n1 * g.n2, half = g.n1 * g.nzc;
@@ -332,6 +335,7 @@ __global__ void __launch_bounds__(NT_MAX) ka_xpass(const __grid_constant__ Plan 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TileBuf<C> sm(smem_raw, g, NBR * TJ);
     const lfts_step_job jb = jobs[blockIdx.y];
+    grid_wait();
     if (jb.active && !jb.active[jb.replica]) return;
     __syncthreads();
     const int plane = g.n1 * g.nzc, j0 = blockIdx.x * TJ, nj = min(TJ, plane - j0);

@@ -171,16 +171,18 @@ __global__ void __launch_bounds__(NT) kf_plane_forward(GridPlan g, const lfts_st
     C *P = (C *)smem_raw;
     C *zl = P + SM::P_ELEMS;
     C *stw = zl + SM::Z_ELEMS;
+    load_stw<C, N, NT>(stw, g.stw);
+    grid_wait();
     const lfts_step_job jb = jobs[blockIdx.y];
     if (jb.active && !jb.active[jb.replica]) return;
     const int x = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    load_stw<C, N, NT>(stw, g.stw);
-    __syncthreads();  // the z transforms below are warp-private but read twiddles that other warps loaded
     const long long poff = (long long)x * N * N;
     const T *qin = (const T *)jb.in + s * jb.in_stride + poff;
     const T *fac = (const T *)jb.fac + poff;
     C *zw = zl + warp * ZB * PL;
-    for (int u0 = warp * ZB; u0 < NU; u0 += (NT / 32) * ZB) {
+    // The z transforms are warp-private but read twiddles that other warps load: every
+    // warp passes one barrier, after it has issued its first rows' loads.
+    for (int u0 = warp * ZB, first = 1; first || u0 < NU; u0 += (NT / 32) * ZB, first = 0) {
         constexpr int PER = (N + 31) / 32;
         T qa[ZB][PER], qb[ZB][PER], fa[ZB][PER], fb[ZB][PER];
 #pragma unroll
@@ -200,6 +202,8 @@ __global__ void __launch_bounds__(NT) kf_plane_forward(GridPlan g, const lfts_st
                 }
             }
         }
+        if (first) __syncthreads();
+        if (u0 >= NU) break;
 #pragma unroll
         for (int b = 0; b < ZB; b++) {
 #pragma unroll
@@ -265,9 +269,10 @@ __global__ void __launch_bounds__(NTHR) kf_xpass(GridPlan g, const lfts_step_job
     C *tile = (C *)smem_raw;
     C *stw = tile + NBR * N * TJ;
     const lfts_step_job jb = jobs[blockIdx.y];
+    load_stw<C, N>(stw, g.stw);
+    grid_wait();
     if (jb.active && !jb.active[jb.replica]) return;
     const int tid = threadIdx.x;
-    load_stw<C, N>(stw, g.stw);
     const long long j0 = (long long)blockIdx.x * TJ;
     const C *spec = (const C *)jb.spec;
     constexpr int TOT = NBR * N * TJ;
@@ -330,9 +335,10 @@ __global__ void __launch_bounds__(NT) kf_plane_mid(GridPlan g, const lfts_step_j
     C *zl = P + SM::P_ELEMS;
     C *stw = zl + SM::Z_ELEMS;
     const lfts_step_job jb = jobs[blockIdx.y];
+    load_stw<C, N, NT>(stw, g.stw);
+    grid_wait();
     if (jb.active && !jb.active[jb.replica]) return;
     const int x = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    load_stw<C, N, NT>(stw, g.stw);
     __syncthreads();
     fload_inverse_y<C, N, 1, NT>(g, jb, spec_idx, P, stw);
     const T *fac = (const T *)jb.fac + (long long)x * N * N;
@@ -418,9 +424,10 @@ __global__ void __launch_bounds__(NT) kf_plane_inverse(GridPlan g, const lfts_st
     C *zl = P + SM::P_ELEMS;
     C *stw = zl + SM::Z_ELEMS;
     const lfts_step_job jb = jobs[blockIdx.y];
+    load_stw<C, N, NT>(stw, g.stw);
+    grid_wait();
     if (jb.active && !jb.active[jb.replica]) return;
     const int x = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    load_stw<C, N, NT>(stw, g.stw);
     __syncthreads();
     fload_inverse_y<C, N, NBR, NT>(g, jb, spec_in0, P, stw);
     const long long poff = (long long)x * N * N;

@@ -274,11 +274,12 @@ __global__ void __launch_bounds__(NTHR, (sizeof(T) == 4 ? LFTS_R8_MINB_F32 : LFT
     constexpr int fm0 = FM0, fm1 = FM1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *P = (C *)smem_raw;
-    const lfts_step_job jb = jobs[blockIdx.y];
-    if (jb.active && !jb.active[jb.replica]) return;
     const int x = blockIdx.x, tid = threadIdx.x, lane = tid & 31, j = lane & 7, grp = tid >> 3;
     const unsigned mask = 0xFFu << (lane & 24);
     const C wf = tw_base<C>(j, -1);
+    grid_wait();
+    const lfts_step_job jb = jobs[blockIdx.y];
+    if (jb.active && !jb.active[jb.replica]) return;
     const long long poff = (long long)x * N * N;
     const T *qin = (const T *)jb.in + s * jb.in_stride + poff;
     const T *fac = (const T *)jb.fac + poff;
@@ -411,6 +412,7 @@ __global__ void __launch_bounds__(NTHR, 3) kp_xpass(GridPlan g, const lfts_step_
     uint64_t *bar = (uint64_t *)(stage + 2 * N * XW);
     const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
     const int nitems = nj * NBR * XTILES;  // < 2^31 for nj <= 65535
+    grid_wait();
     // first item at or after it whose job is active and aligned (>= nitems: none)
     auto next_item = [&](int it) -> int {
         for (; it < nitems; it += (int)gridDim.x) {
@@ -507,10 +509,11 @@ __global__ void __launch_bounds__(NTHR, (sizeof(T) == 4 ? LFTS_R8_MINB_F32 : LFT
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *P = (C *)smem_raw;
     const lfts_step_job jb = jobs[blockIdx.y];
-    if (jb.active && !jb.active[jb.replica]) return;
     const int x = blockIdx.x, tid = threadIdx.x, lane = tid & 31, j = lane & 7, grp = tid >> 3;
     const unsigned mask = 0xFFu << (lane & 24);
     const C wf = tw_base<C>(j, -1), wi = tw_base<C>(j, +1);
+    grid_wait();
+    if (jb.active && !jb.active[jb.replica]) return;
     C *sp = (C *)jb.spec + (size_t)spec_idx * g.Mc + (size_t)x * PLANE;
     const T *fac = (const T *)jb.fac + (long long)x * N * N;
     y_inverse_paired(P, grp, j, wi, mask, sp);
@@ -554,10 +557,11 @@ __global__ void __launch_bounds__(NTHR, (sizeof(T) == 4 ? LFTS_R8_MINB_F32 : LFT
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *P = (C *)smem_raw;
     const lfts_step_job jb = jobs[blockIdx.y];
-    if (jb.active && !jb.active[jb.replica]) return;
     const int x = blockIdx.x, tid = threadIdx.x, lane = tid & 31, j = lane & 7, grp = tid >> 3;
     const unsigned mask = 0xFFu << (lane & 24);
     const C wi = tw_base<C>(j, +1);
+    grid_wait();
+    if (jb.active && !jb.active[jb.replica]) return;
     const C *in = (const C *)jb.spec + (size_t)spec_in0 * g.Mc + (size_t)x * PLANE;
     const long long poff = (long long)x * N * N;
     const T *fac = (const T *)jb.fac + poff;
