@@ -1611,38 +1611,34 @@ extern "C" int lfts_realspace_tables(lfts_ctx c, double b2, double ds, int dim, 
     return 0;
 }
 
+// 32 lines a block while the tile leaves room for two blocks on an SM (n <= 330), else 16
+template <int DIM, int A, bool FIRST, bool LAST>
+static int rs_sweep(lfts_ctx c, const lfts_step_job *jobs, int nj, int s, int src_half) {
+    const int n = A == 0 ? c->g.n0 : A == 1 ? c->g.n1 : c->g.n2;
+    const bool wide = rs::tile_smem(n, 32) <= 110 * 1024;
+    const int W = wide ? 32 : 16;
+    const size_t smem = rs::tile_smem(n, W);
+    const dim3 grid((unsigned)((c->g.M / n + W - 1) / W), nj);
+    auto kernel = wide ? rs::k_rs_sweep<DIM, A, FIRST, LAST, 32> : rs::k_rs_sweep<DIM, A, FIRST, LAST, 16>;
+    if (smem > 48 * 1024) CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CK(launch_after(kernel, grid, dim3(rs::NT), smem, c->stream, c->g, jobs, s, src_half));
+    c->launches += 1;
+    return 0;
+}
 extern "C" int lfts_step_realspace(lfts_ctx c, const lfts_step_job *jobs, int nj, int s, int dim) {
     if (!c || !jobs) return fail("null argument");
     if (c->prec != 8) return fail("the real-space step runs in FP64 contexts only");
     if (dim < 1 || dim > 3 || dim != c->dim) return fail("real-space step: dim must be the context's dimension");
     if (nj <= 0) return 0;
     if (nj > 65535) return fail("real-space step: at most 65535 jobs per call");
-    const GridPlan &g = c->g;
-    cudaStream_t st = c->stream;
-    auto blocks = [&](long long n_axis) { return (unsigned)((g.M / n_axis + NTHR - 1) / NTHR); };
-    // the last-axis sweep through a shared-memory tile of ZL lines
-    // (a tile of long lines that does not fit shared memory walks the lines in global memory)
-    const size_t zsm = sizeof(double) * 2 * rs::ZL * (size_t)(g.n2 + 1);
-    const unsigned zblocks = (unsigned)((g.M / g.n2 + rs::ZL - 1) / rs::ZL);
-    const bool tiled = zsm <= 200 * 1024;
-    if (tiled && zsm > 48 * 1024)
-        CK(cudaFuncSetAttribute(rs::k_rs_last_axis<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsm));
-    auto last_axis = [&](int src_half) {
-        if (tiled) rs::k_rs_last_axis<true><<<dim3(zblocks, nj), rs::ZL, zsm, st>>>(g, jobs, s, src_half);
-        else rs::k_rs_next<2, true><<<dim3(blocks(g.n2), nj), NTHR, 0, st>>>(g, jobs, s, src_half);
-    };
     if (dim == 3) {
-        rs::k_rs_first<3><<<dim3(blocks(g.n0), nj), NTHR, 0, st>>>(g, jobs, s);
-        rs::k_rs_next<1, false><<<dim3(blocks(g.n1), nj), NTHR, 0, st>>>(g, jobs, s, 0);
-        last_axis(1);
-        c->launches += 3;
+        if (rs_sweep<3, 0, true, false>(c, jobs, nj, s, 0) || rs_sweep<3, 1, false, false>(c, jobs, nj, s, 0) ||
+            rs_sweep<3, 2, false, true>(c, jobs, nj, s, 1))
+            return -1;
     } else if (dim == 2) {
-        rs::k_rs_first<2><<<dim3(blocks(g.n1), nj), NTHR, 0, st>>>(g, jobs, s);
-        last_axis(0);
-        c->launches += 2;
-    } else {
-        rs::k_rs_first<1><<<dim3(blocks(g.n2), nj), NTHR, 0, st>>>(g, jobs, s);
-        c->launches += 1;
+        if (rs_sweep<2, 1, true, false>(c, jobs, nj, s, 0) || rs_sweep<2, 2, false, true>(c, jobs, nj, s, 0)) return -1;
+    } else if (rs_sweep<1, 2, true, true>(c, jobs, nj, s, 0)) {
+        return -1;
     }
     CKLAUNCH();
     return 0;
