@@ -519,6 +519,37 @@ extern "C" int lfts_graph_destroy(lfts_graph g) {
 // ---------------------------------------------------------------- tables
 // Boltzmann bond factor, same arithmetic as the reference's Pseudo.cpp:17-82
 // (xfactor from nx*dx, integer wave numbers folded at n/2), then / M.
+// On the device: a relaxing box rebuilds them every SCFT iteration, and 5e5
+// exponentials a monomer type on the host took more time than the propagators (64^3).
+__device__ __forceinline__ void wave_numbers(const GridPlan &g, long long idx, int &i, int &j, int &k) {
+    const long long r = idx / g.nzc;
+    k = (int)(idx - r * g.nzc);
+    i = (int)(r / g.n1);
+    j = (int)(r - (long long)i * g.n1);
+    if (i > g.n0 / 2) i = g.n0 - i;
+    if (j > g.n1 / 2) j = g.n1 - j;
+}
+template <typename T>
+__global__ void __launch_bounds__(NTHR) k_bond_tables(GridPlan g, double3 xf, double3 xh, double inv_m, T *__restrict__ b,
+                                                      T *__restrict__ bh) {
+    for (long long idx = blockIdx.x * (long long)NTHR + threadIdx.x; idx < g.Mc; idx += (long long)gridDim.x * NTHR) {
+        int i, j, k;
+        wave_numbers(g, idx, i, j, k);
+        b[idx] = (T)(exp(i * i * xf.x + j * j * xf.y + k * k * xf.z) * inv_m);
+        bh[idx] = (T)(exp(i * i * xh.x + j * j * xh.y + k * k * xh.z) * inv_m);
+    }
+}
+__global__ void __launch_bounds__(NTHR) k_fourier_basis(GridPlan g, double3 xf, double *__restrict__ basis) {
+    for (long long idx = blockIdx.x * (long long)NTHR + threadIdx.x; idx < g.Mc; idx += (long long)gridDim.x * NTHR) {
+        int i, j, k;
+        wave_numbers(g, idx, i, j, k);
+        const double twice = (k != 0 && 2 * k != g.n2) ? 2.0 : 1.0;
+        basis[idx] = i * i * xf.x * twice;
+        basis[g.Mc + idx] = j * j * xf.y * twice;
+        basis[2 * g.Mc + idx] = k * k * xf.z * twice;
+    }
+}
+static int grid_for(long long n);
 template <typename T>
 static int bond_tables_t(lfts_ctx c, double b2, double ds, const double *lx, void *b_out, void *bh_out) {
     const GridPlan &g = c->g;
@@ -526,26 +557,15 @@ static int bond_tables_t(lfts_ctx c, double b2, double ds, const double *lx, voi
     double tdx[3] = {1.0, 1.0, 1.0};
     for (int d = 0; d < c->dim; d++) tdx[3 - c->dim + d] = lx[d] / c->nx[3 - c->dim + d];
     const double PI = 3.14159265358979323846;
-    std::vector<T> hb(g.Mc), hh(g.Mc);
-    double xf[3], xh[3];
+    double3 xf, xh;
+    double *f = &xf.x, *h = &xh.x;
     for (int d = 0; d < 3; d++) {
-        xf[d] = -b2 * std::pow(2 * PI / (tn[d] * tdx[d]), 2) * ds / 6.0;
-        xh[d] = -(b2 / 2) * std::pow(2 * PI / (tn[d] * tdx[d]), 2) * ds / 6.0;
+        f[d] = -b2 * std::pow(2 * PI / (tn[d] * tdx[d]), 2) * ds / 6.0;
+        h[d] = -(b2 / 2) * std::pow(2 * PI / (tn[d] * tdx[d]), 2) * ds / 6.0;
     }
-    const double invM = 1.0 / (double)g.M;
-    for (int i = 0; i < tn[0]; i++) {
-        const int it = i > tn[0] / 2 ? tn[0] - i : i;
-        for (int j = 0; j < tn[1]; j++) {
-            const int jt = j > tn[1] / 2 ? tn[1] - j : j;
-            for (int k = 0; k < g.nzc; k++) {
-                const long long idx = ((long long)i * tn[1] + j) * g.nzc + k;
-                hb[idx] = (T)(std::exp(it * it * xf[0] + jt * jt * xf[1] + k * k * xf[2]) * invM);
-                hh[idx] = (T)(std::exp(it * it * xh[0] + jt * jt * xh[1] + k * k * xh[2]) * invM);
-            }
-        }
-    }
-    CK(cudaMemcpyAsync(b_out, hb.data(), sizeof(T) * g.Mc, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(bh_out, hh.data(), sizeof(T) * g.Mc, cudaMemcpyHostToDevice, c->stream));
+    k_bond_tables<T><<<grid_for(g.Mc), NTHR, 0, c->stream>>>(g, xf, xh, 1.0 / (double)g.M, (T *)b_out, (T *)bh_out);
+    c->launches += 1;
+    CKLAUNCH();
     CK(cudaStreamSynchronize(c->stream));
     return 0;
 }
@@ -563,24 +583,11 @@ extern "C" int lfts_fourier_basis(lfts_ctx c, const double *lx, double *basis_ou
     double tdx[3] = {1.0, 1.0, 1.0};
     for (int d = 0; d < c->dim; d++) tdx[3 - c->dim + d] = lx[d] / c->nx[3 - c->dim + d];
     const double PI = 3.14159265358979323846;
-    double xf[3];
-    for (int d = 0; d < 3; d++) xf[d] = std::pow(2 * PI / (tn[d] * tdx[d]), 2);
-    std::vector<double> h(3 * g.Mc);
-    for (int i = 0; i < tn[0]; i++) {
-        const int it = i > tn[0] / 2 ? tn[0] - i : i;
-        for (int j = 0; j < tn[1]; j++) {
-            const int jt = j > tn[1] / 2 ? tn[1] - j : j;
-            for (int k = 0; k < g.nzc; k++) {
-                const long long idx = ((long long)i * tn[1] + j) * g.nzc + k;
-                double bx = it * it * xf[0], by = jt * jt * xf[1], bz = k * k * xf[2];
-                if (k != 0 && 2 * k != tn[2]) { bx *= 2; by *= 2; bz *= 2; }
-                h[idx] = bx;
-                h[g.Mc + idx] = by;
-                h[2 * g.Mc + idx] = bz;
-            }
-        }
-    }
-    CK(cudaMemcpyAsync(basis_out, h.data(), sizeof(double) * 3 * g.Mc, cudaMemcpyHostToDevice, c->stream));
+    const double3 xf = make_double3(std::pow(2 * PI / (tn[0] * tdx[0]), 2), std::pow(2 * PI / (tn[1] * tdx[1]), 2),
+                                    std::pow(2 * PI / (tn[2] * tdx[2]), 2));
+    k_fourier_basis<<<grid_for(g.Mc), NTHR, 0, c->stream>>>(g, xf, basis_out);
+    c->launches += 1;
+    CKLAUNCH();
     CK(cudaStreamSynchronize(c->stream));
     return 0;
 }
@@ -1000,6 +1007,30 @@ __global__ void k_stress_prep(const lfts_stress_job *__restrict__ jobs, int nj, 
     }
 }
 
+// zy spectra of one field per job into slot 0 by the context's own forward plane kernel
+template <typename T, int N> static void planes_forward_fast(lfts_ctx c, const lfts_step_job *jobs, int nj) {
+    using C = typename CT<T>::type;
+    const dim3 grid(N, nj);
+    if constexpr (N == r8::N) {
+        if (c->r8) {
+            r8::kr_plane_forward<T, 1, FM_NONE, FM_NONE><<<grid, NTHR, r8::plane_smem<C>(), c->stream>>>(c->g, jobs, 0, 0);
+            return;
+        }
+    }
+    fast::kf_plane_forward<T, 1, N><<<grid, NTHR, fast::FSmem<C, N, 1, 1>::BYTES, c->stream>>>(c->g, jobs, 0, FM_NONE, 0, 0);
+}
+template <typename T> static void planes_forward(lfts_ctx c, const lfts_step_job *jobs, int nj) {
+    switch (c->fastN) {
+        case 16: return planes_forward_fast<T, 16>(c, jobs, nj);
+        case 32: return planes_forward_fast<T, 32>(c, jobs, nj);
+        case 48: return planes_forward_fast<T, 48>(c, jobs, nj);
+        case 64: return planes_forward_fast<T, 64>(c, jobs, nj);
+        case 96: return planes_forward_fast<T, 96>(c, jobs, nj);
+        case 128: return planes_forward_fast<T, 128>(c, jobs, nj);
+    }
+    any_planes_forward(c->any, c->stream, jobs, nj);
+}
+
 template <typename T, bool GEN>
 static int stress_t(lfts_ctx c, const lfts_stress_job *jobs, int nj, const double *basis, void *spec, int max_chunk,
                     double *out) {
@@ -1013,7 +1044,7 @@ static int stress_t(lfts_ctx c, const lfts_stress_job *jobs, int nj, const doubl
         if ((size_t)n * ntiles * 3 > c->partials_cap) return fail("stress chunk exceeds the partial-sum workspace");
         k_stress_prep<T><<<(n + 127) / 128, 128, 0, st>>>(jobs + j0, n, spec, g.Mc, c->sjobs);
         if (c->any) {
-            any_planes_forward(c->any, st, c->sjobs, 2 * n);
+            planes_forward<T>(c, c->sjobs, 2 * n);
             any_xstress(c->any, st, c->sjobs, jobs + j0, n, basis, c->partials);
         } else {
             k_plane_forward<T, 1, GEN><<<dim3(g.n0, 2 * n), NTHR, c->sm_pf1, st>>>(g, c->sjobs, 0, FM_NONE, 0, 0, c->zb);
