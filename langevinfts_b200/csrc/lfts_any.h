@@ -15,7 +15,7 @@ struct AnyGrid;  // plan, device tables and launch limits of one grid and precis
 AnyGrid *any_create(int prec, const int n[3], int nsm, int max_smem, std::string &err);
 void any_destroy(AnyGrid *a);
 
-void any_step_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s);
+void any_steps_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps);
 void any_step_discrete(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s, int half, int with_fac);
 // zy-transforms of one real field per job into spectrum slot 0 (half the 3D transform)
 void any_planes_forward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj);
@@ -29,7 +29,7 @@ void any_xstress(const AnyGrid *a, cudaStream_t st, const lfts_step_job *sj, con
 
 // CTAs per job of the cluster sweep for nj jobs; 0: the grid does not fit or the
 // separate passes are faster.  force: 0 by that rule, else this cluster size where it fits.
-int any_sweep_size(const AnyGrid *a, bool continuous, int nj, int force);
+int any_sweep_size(AnyGrid *a, bool continuous, int nj, int force);
 int any_sweep_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps, int cs);
 int any_sweep_discrete(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps, int half,
                        int with_fac, int cs);

@@ -159,6 +159,7 @@ template <typename T, int N> static int fast_setup(int max_smem) {
     if (allow_smem(fast::kf_plane_mid<T, N>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(fast::kf_plane_inverse<T, 2, EPI_RICH, N, NT2>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(fast::kf_plane_inverse<T, 1, EPI_SCALE, N>, max_smem) != cudaSuccess) return 0;
+    if (allow_smem(fast::kf_plane_seam<T, N, NT2>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(fast::kf_xpass<T, 1, N>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(fast::kf_xpass<T, 2, N>, max_smem) != cudaSuccess) return 0;
     (void)f1;
@@ -171,6 +172,9 @@ template <typename T> static int r12_setup(int max_smem) {
     if (allow_smem(r12::kq_plane_forward<T, FM_FAC_SQ, FM_FAC>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(r12::kq_plane_mid<T>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(r12::kq_plane_inverse<T>, max_smem) != cudaSuccess) return 0;
+    if constexpr (sizeof(T) == 8) {
+        if (allow_smem(r12::kq_plane_seam<T>, max_smem) != cudaSuccess) return 0;
+    }
     if (allow_smem(r12::kq_xpass<T, 1>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(r12::kq_xpass<T, 2>, max_smem) != cudaSuccess) return 0;
     return 1;
@@ -184,6 +188,7 @@ template <typename T> static int r8_setup(int max_smem) {
     if (allow_smem(r8::kr_plane_mid<T>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(r8::kr_plane_inverse<T, 2, EPI_RICH>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(r8::kr_plane_inverse<T, 1, EPI_SCALE>, max_smem) != cudaSuccess) return 0;
+    if (allow_smem(r8::kr_plane_seam<T>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(r8::kp_xpass<T, 1>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(r8::kp_xpass<T, 2>, max_smem) != cudaSuccess) return 0;
     return 1;
@@ -614,11 +619,14 @@ extern "C" int lfts_field_factors(lfts_ctx c, const double *w, double coef, void
 }
 
 // ---------------------------------------------------------------- steps
+// Steps s0 .. s0 + nsteps - 1, each from what the one before wrote: K1, then per step
+// K2, K3, K4 and the seam to the next, K5 after the last.
 template <typename T, int N>
-static int step_cont_fast(lfts_ctx c, const lfts_step_job *jobs, int nj, int s) {
+static int steps_cont_fast(lfts_ctx c, const lfts_step_job *jobs, int nj, int s0, int nsteps) {
     using C = typename CT<T>::type;
     const GridPlan &g = c->g;
     cudaStream_t st = c->stream;
+    const int last = s0 + nsteps - 1;
     constexpr int TJ = sizeof(T) == 8 ? 16 : 32;
     const dim3 gp(N, nj), gx((unsigned)(((long long)N * (N / 2 + 1) + TJ - 1) / TJ), nj);
     constexpr int NT2 = fast_nt2<T, N>();
@@ -631,11 +639,14 @@ static int step_cont_fast(lfts_ctx c, const lfts_step_job *jobs, int nj, int s) 
             const size_t ps = r8::plane_smem<C>();
             const long long it2 = (long long)nj * 2 * r8::xpipe_tiles<C>(), it1 = (long long)nj * r8::xpipe_tiles<C>(), cap = (long long)(c->xcap ? c->xcap : 3) * c->nsm;
             const dim3 px2((unsigned)(it2 < cap ? it2 : cap)), px1((unsigned)(it1 < cap ? it1 : cap));
-            CK(launch_after(r8::kr_plane_forward<T, 2, FM_FAC_SQ, FM_FAC>, dim3(rp), NTHR, ps, st, g, jobs, s, 0));
-            CK(launch_after(r8::kp_xpass<T, 2>, dim3(px2), NTHR, r8::xpipe_smem<C>(), st, g, jobs, nj, 0, 0, 1));
-            CK(launch_after(r8::kr_plane_mid<T>, dim3(rp), NTHR, ps, st, g, jobs, 1));
-            CK(launch_after(r8::kp_xpass<T, 1>, dim3(px1), NTHR, r8::xpipe_smem<C>(), st, g, jobs, nj, 1, 1, 1));
-            CK(launch_after(r8::kr_plane_inverse<T, 2, EPI_RICH>, dim3(rp), NTHR, ps, st, g, jobs, s, 0, 0));
+            CK(launch_after(r8::kr_plane_forward<T, 2, FM_FAC_SQ, FM_FAC>, dim3(rp), NTHR, ps, st, g, jobs, s0, 0));
+            for (int s = s0; s <= last; s++) {
+                CK(launch_after(r8::kp_xpass<T, 2>, dim3(px2), NTHR, r8::xpipe_smem<C>(), st, g, jobs, nj, 0, 0, 1));
+                CK(launch_after(r8::kr_plane_mid<T>, dim3(rp), NTHR, ps, st, g, jobs, 1));
+                CK(launch_after(r8::kp_xpass<T, 1>, dim3(px1), NTHR, r8::xpipe_smem<C>(), st, g, jobs, nj, 1, 1, 1));
+                if (s < last) CK(launch_after(r8::kr_plane_seam<T>, dim3(rp), NTHR, ps, st, g, jobs, s));
+                else CK(launch_after(r8::kr_plane_inverse<T, 2, EPI_RICH>, dim3(rp), NTHR, ps, st, g, jobs, s, 0, 0));
+            }
             CKLAUNCH();
             return 0;
         }
@@ -645,20 +656,33 @@ static int step_cont_fast(lfts_ctx c, const lfts_step_job *jobs, int nj, int s) 
             const size_t p2 = r12::plane_smem<C>(N), p1 = r12::plane_smem<C>(N / 2), xs = r12::xpipe_smem<C>();
             const long long it2 = (long long)nj * 2 * r12::XTILES, it1 = (long long)nj * r12::XTILES;
             const long long cap = (long long)(c->xcap ? c->xcap : r12::minb_xpass<T>()) * c->nsm;
-            CK(launch_after(r12::kq_plane_forward<T, FM_FAC_SQ, FM_FAC>, dim3(gp), r12::NT, p2, st, g, jobs, s, 0));
-            CK(launch_after(r12::kq_xpass<T, 2>, dim3((unsigned)(it2 < cap ? it2 : cap)), NTHR, xs, st, g, jobs, nj, 0, 0, 1));
-            CK(launch_after(r12::kq_plane_mid<T>, dim3(gp), r12::NT, p1, st, g, jobs, 1));
-            CK(launch_after(r12::kq_xpass<T, 1>, dim3((unsigned)(it1 < cap ? it1 : cap)), NTHR, xs, st, g, jobs, nj, 1, 1, 1));
-            CK(launch_after(r12::kq_plane_inverse<T>, dim3(gp), r12::NT, p2, st, g, jobs, s, 0));
+            CK(launch_after(r12::kq_plane_forward<T, FM_FAC_SQ, FM_FAC>, dim3(gp), r12::NT, p2, st, g, jobs, s0, 0));
+            for (int s = s0; s <= last; s++) {
+                CK(launch_after(r12::kq_xpass<T, 2>, dim3((unsigned)(it2 < cap ? it2 : cap)), NTHR, xs, st, g, jobs, nj, 0, 0, 1));
+                CK(launch_after(r12::kq_plane_mid<T>, dim3(gp), r12::NT, p1, st, g, jobs, 1));
+                CK(launch_after(r12::kq_xpass<T, 1>, dim3((unsigned)(it1 < cap ? it1 : cap)), NTHR, xs, st, g, jobs, nj, 1, 1, 1));
+                if constexpr (sizeof(T) == 8) {
+                    if (s < last) {
+                        CK(launch_after(r12::kq_plane_seam<T>, dim3(gp), r12::NT, p2, st, g, jobs, s));
+                        continue;
+                    }
+                }
+                CK(launch_after(r12::kq_plane_inverse<T>, dim3(gp), r12::NT, p2, st, g, jobs, s, 0));
+                // FP32: the seam's two transforms spill at two CTAs an SM (210 against 208 us a step, 8 jobs)
+                if (sizeof(T) == 4 && s < last) CK(launch_after(r12::kq_plane_forward<T, FM_FAC_SQ, FM_FAC>, dim3(gp), r12::NT, p2, st, g, jobs, s + 1, 0));
+            }
             CKLAUNCH();
             return 0;
         }
     }
-    CK(launch_after(fast::kf_plane_forward<T, 2, N, NT2>, dim3(gp), NT2, f2, st, g, jobs, s, FM_FAC_SQ, FM_FAC, 0));
-    CK(launch_after(fast::kf_xpass<T, 2, N>, dim3(gx), NTHR, x2, st, g, jobs, 0, 0, 1));
-    CK(launch_after(fast::kf_plane_mid<T, N>, dim3(gp), NTHR, f1, st, g, jobs, 1));
-    CK(launch_after(fast::kf_xpass<T, 1, N>, dim3(gx), NTHR, x1, st, g, jobs, 1, 1, 1));
-    CK(launch_after(fast::kf_plane_inverse<T, 2, EPI_RICH, N, NT2>, dim3(gp), NT2, f2, st, g, jobs, s, 0, 0));
+    CK(launch_after(fast::kf_plane_forward<T, 2, N, NT2>, dim3(gp), NT2, f2, st, g, jobs, s0, FM_FAC_SQ, FM_FAC, 0));
+    for (int s = s0; s <= last; s++) {
+        CK(launch_after(fast::kf_xpass<T, 2, N>, dim3(gx), NTHR, x2, st, g, jobs, 0, 0, 1));
+        CK(launch_after(fast::kf_plane_mid<T, N>, dim3(gp), NTHR, f1, st, g, jobs, 1));
+        CK(launch_after(fast::kf_xpass<T, 1, N>, dim3(gx), NTHR, x1, st, g, jobs, 1, 1, 1));
+        if (s < last) CK(launch_after(fast::kf_plane_seam<T, N, NT2>, dim3(gp), NT2, f2, st, g, jobs, s));
+        else CK(launch_after(fast::kf_plane_inverse<T, 2, EPI_RICH, N, NT2>, dim3(gp), NT2, f2, st, g, jobs, s, 0, 0));
+    }
     CKLAUNCH();
     return 0;
 }
@@ -690,14 +714,14 @@ static int step_disc_fast(lfts_ctx c, const lfts_step_job *jobs, int nj, int s, 
     return 0;
 }
 template <typename T>
-static int step_fast_dispatch(lfts_ctx c, const lfts_step_job *jobs, int nj, int s, int disc, int half, int wf) {
+static int step_fast_dispatch(lfts_ctx c, const lfts_step_job *jobs, int nj, int s, int nsteps, int disc, int half, int wf) {
     switch (c->fastN) {
-        case 16: return disc ? step_disc_fast<T, 16>(c, jobs, nj, s, half, wf) : step_cont_fast<T, 16>(c, jobs, nj, s);
-        case 32: return disc ? step_disc_fast<T, 32>(c, jobs, nj, s, half, wf) : step_cont_fast<T, 32>(c, jobs, nj, s);
-        case 48: return disc ? step_disc_fast<T, 48>(c, jobs, nj, s, half, wf) : step_cont_fast<T, 48>(c, jobs, nj, s);
-        case 64: return disc ? step_disc_fast<T, 64>(c, jobs, nj, s, half, wf) : step_cont_fast<T, 64>(c, jobs, nj, s);
-        case 96: return disc ? step_disc_fast<T, 96>(c, jobs, nj, s, half, wf) : step_cont_fast<T, 96>(c, jobs, nj, s);
-        case 128: return disc ? step_disc_fast<T, 128>(c, jobs, nj, s, half, wf) : step_cont_fast<T, 128>(c, jobs, nj, s);
+        case 16: return disc ? step_disc_fast<T, 16>(c, jobs, nj, s, half, wf) : steps_cont_fast<T, 16>(c, jobs, nj, s, nsteps);
+        case 32: return disc ? step_disc_fast<T, 32>(c, jobs, nj, s, half, wf) : steps_cont_fast<T, 32>(c, jobs, nj, s, nsteps);
+        case 48: return disc ? step_disc_fast<T, 48>(c, jobs, nj, s, half, wf) : steps_cont_fast<T, 48>(c, jobs, nj, s, nsteps);
+        case 64: return disc ? step_disc_fast<T, 64>(c, jobs, nj, s, half, wf) : steps_cont_fast<T, 64>(c, jobs, nj, s, nsteps);
+        case 96: return disc ? step_disc_fast<T, 96>(c, jobs, nj, s, half, wf) : steps_cont_fast<T, 96>(c, jobs, nj, s, nsteps);
+        case 128: return disc ? step_disc_fast<T, 128>(c, jobs, nj, s, half, wf) : steps_cont_fast<T, 128>(c, jobs, nj, s, nsteps);
     }
     return fail("no specialised kernels for this grid");
 }
@@ -727,23 +751,31 @@ static int step_cont_t(lfts_ctx c, const lfts_step_job *jobs, int nj, int s) {
     CKLAUNCH();
     return 0;
 }
+static int steps_continuous(lfts_ctx c, const lfts_step_job *jobs, int nj, int s0, int nsteps) {
+    if (c->fastN) {
+        c->launches += c->r12 && c->prec == 4 ? 5 * (long long)nsteps : 1 + 4 * (long long)nsteps;
+        return c->prec == 8 ? step_fast_dispatch<double>(c, jobs, nj, s0, nsteps, 0, 0, 0)
+                            : step_fast_dispatch<float>(c, jobs, nj, s0, nsteps, 0, 0, 0);
+    }
+    if (c->any) {
+        c->launches += 1 + 4 * (long long)nsteps;
+        any_steps_continuous(c->any, c->stream, jobs, nj, s0, nsteps);
+        CKLAUNCH();
+        return 0;
+    }
+    for (int s = s0; s < s0 + nsteps; s++) {
+        c->launches += c->nbr2 ? 5 : 8;
+        const int rc = c->prec == 8 ? (c->gen ? step_cont_t<double, true>(c, jobs, nj, s) : step_cont_t<double, false>(c, jobs, nj, s))
+                                    : (c->gen ? step_cont_t<float, true>(c, jobs, nj, s) : step_cont_t<float, false>(c, jobs, nj, s));
+        if (rc) return rc;
+    }
+    return 0;
+}
 extern "C" int lfts_step_continuous(lfts_ctx c, const lfts_step_job *jobs, int nj, int s) {
     if (!c || !jobs) return fail("null argument");
     if (nj <= 0) return 0;
     if (nj > 65535) return fail("too many jobs in one launch (max 65535)");
-    if (c->fastN) {
-        c->launches += 5;
-        return c->prec == 8 ? step_fast_dispatch<double>(c, jobs, nj, s, 0, 0, 0) : step_fast_dispatch<float>(c, jobs, nj, s, 0, 0, 0);
-    }
-    if (c->any) {
-        c->launches += 5;
-        any_step_continuous(c->any, c->stream, jobs, nj, s);
-        CKLAUNCH();
-        return 0;
-    }
-    c->launches += c->nbr2 ? 5 : 8;
-    if (c->prec == 8) return c->gen ? step_cont_t<double, true>(c, jobs, nj, s) : step_cont_t<double, false>(c, jobs, nj, s);
-    return c->gen ? step_cont_t<float, true>(c, jobs, nj, s) : step_cont_t<float, false>(c, jobs, nj, s);
+    return steps_continuous(c, jobs, nj, s, 1);
 }
 
 template <typename T, bool GEN>
@@ -764,8 +796,8 @@ extern "C" int lfts_step_discrete(lfts_ctx c, const lfts_step_job *jobs, int nj,
     half = half ? 1 : 0;
     c->launches += 3;
     if (c->fastN)
-        return c->prec == 8 ? step_fast_dispatch<double>(c, jobs, nj, s, 1, half, with_fac)
-                            : step_fast_dispatch<float>(c, jobs, nj, s, 1, half, with_fac);
+        return c->prec == 8 ? step_fast_dispatch<double>(c, jobs, nj, s, 1, 1, half, with_fac)
+                            : step_fast_dispatch<float>(c, jobs, nj, s, 1, 1, half, with_fac);
     if (c->any) {
         any_step_discrete(c->any, c->stream, jobs, nj, s, half, with_fac);
         CKLAUNCH();
@@ -793,11 +825,7 @@ extern "C" int lfts_sweep_continuous(lfts_ctx c, const lfts_step_job *jobs, int 
         c->launches += 1;
         return 0;
     }
-    for (int s = s0; s < s0 + nsteps; s++) {
-        const int rc = lfts_step_continuous(c, jobs, nj, s);
-        if (rc) return rc;
-    }
-    return 0;
+    return steps_continuous(c, jobs, nj, s0, nsteps);
 }
 extern "C" int lfts_sweep_discrete(lfts_ctx c, const lfts_step_job *jobs, int nj, int s0, int nsteps, int half, int with_fac) {
     if (!c || !jobs) return fail("null argument");

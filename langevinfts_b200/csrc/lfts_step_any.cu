@@ -14,7 +14,10 @@ struct AnyGrid {
     any::Plan p;
     int prec = 8, nsm = 148, max_smem = 0;
     void *tables = nullptr;
-    int clusters_cont[5] = {0, 0, 0, 0, 0}, clusters_disc[5] = {0, 0, 0, 0, 0};  // resident clusters of 1, 2, 4, 8, 16 CTAs (0: no fit)
+    // resident clusters of 1, 2, 4, 8, 16 CTAs, estimated (0: no fit); the device's own
+    // answer is asked for once, for a size about to be used: it takes a third of a millisecond
+    int clusters_cont[5] = {0, 0, 0, 0, 0}, clusters_disc[5] = {0, 0, 0, 0, 0};
+    bool asked_cont[5] = {}, asked_disc[5] = {};
 };
 
 namespace {
@@ -97,7 +100,7 @@ template <typename K> bool allow(K kernel, int max_smem, bool cluster = false) {
 template <typename T> bool allow_all(int max_smem) {
     return allow(any::ka_plane_forward<T, true>, max_smem) && allow(any::ka_plane_forward<T, false>, max_smem) &&
            allow(any::ka_plane_mid<T>, max_smem) && allow(any::ka_plane_inverse<T, true>, max_smem) &&
-           allow(any::ka_plane_inverse<T, false>, max_smem) && allow(any::ka_xpass<T, 1>, max_smem) &&
+           allow(any::ka_plane_inverse<T, false>, max_smem) && allow(any::ka_plane_seam<T>, max_smem) && allow(any::ka_xpass<T, 1>, max_smem) &&
            allow(any::ka_xpass<T, 2>, max_smem) && allow(any::ka_xpass_forward<T>, max_smem) && allow(any::ka_xstress<T>, max_smem) &&
            allow(any::ka_sweep_continuous<T>, max_smem, true) && allow(any::ka_sweep_discrete<T>, max_smem, true);
 }
@@ -150,7 +153,6 @@ template <typename K> void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAtt
 
 template <typename K> int resident_clusters(const AnyGrid *a, K kernel, bool continuous, int cs) {
     const SweepShape s = sweep_shape(a, continuous, cs);
-    if (s.smem > (size_t)a->max_smem) return 0;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at;
     cluster_config(cfg, &at, kernel, cs, 64, sweep_threads(a, s), s.smem, 0);
@@ -160,6 +162,13 @@ template <typename K> int resident_clusters(const AnyGrid *a, K kernel, bool con
         return 0;
     }
     return n;
+}
+// clusters stay within one of eight groups of SMs; a CTA takes its threads' 128 registers
+int estimate_clusters(const AnyGrid *a, bool continuous, int cs) {
+    const SweepShape s = sweep_shape(a, continuous, cs);
+    if (s.smem > (size_t)a->max_smem) return 0;
+    const int per_sm = (int)std::min<size_t>(512 / sweep_threads(a, s), (size_t)a->max_smem / s.smem);
+    return std::max(1, 8 * (a->nsm / 8 * std::max(per_sm, 1) / cs));
 }
 
 template <typename T> bool setup(AnyGrid *a, std::string &err) {
@@ -197,8 +206,8 @@ template <typename T> bool setup(AnyGrid *a, std::string &err) {
         return false;
     }
     for (int k = 0; k < 5; k++) {
-        a->clusters_cont[k] = resident_clusters(a, any::ka_sweep_continuous<T>, true, 1 << k);
-        a->clusters_disc[k] = resident_clusters(a, any::ka_sweep_discrete<T>, false, 1 << k);
+        a->clusters_cont[k] = estimate_clusters(a, true, 1 << k);
+        a->clusters_disc[k] = estimate_clusters(a, false, 1 << k);
     }
     return true;
 }
@@ -251,15 +260,23 @@ template <typename T, int NBR> void xpass(const AnyGrid *a, cudaStream_t st, con
     const int tj = tile_columns<C>(a, NBR, nj), ctas = ceil_div(g.n1 * g.nzc, tj);
     launch_after(any::ka_xpass<T, NBR>, dim3(ctas, nj), plane_threads(a, ctas * nj, g.n0 * tj * NBR), any::TileBuf<C>::bytes(g, NBR * tj), st, g, jobs, spec, b0, b1, tj, any::div_mul(tj), any::div_mul(NBR * tj));
 }
-template <typename T> void step_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s) {
+template <typename T> void steps_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps) {
     using C = typename CT<T>::type;
     const Plan &g = a->p;
-    plane_forward<T, true>(a, st, jobs, nj, s, FM_FAC_SQ, FM_FAC, 0);
-    xpass<T, 2>(a, st, jobs, nj, 0, 0, 1);
-    const int units = ceil_div(g.n0, 2), k = stack_planes<C>(a, units, nj), ctas = ceil_div(units, k);
-    launch_after(any::ka_plane_mid<T>, dim3(ctas, nj), plane_threads(a, ctas * nj, k * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, k), st, g, jobs, 1, stack(g, k));
-    xpass<T, 1>(a, st, jobs, nj, 1, 1, 1);
-    plane_inverse<T, true>(a, st, jobs, nj, s, 0, 0);
+    const int pairs = ceil_div(g.n0, 2), km = stack_planes<C>(a, pairs, nj), mid_ctas = ceil_div(pairs, km);
+    const int k = stack_planes<C>(a, g.n0, nj), ctas = ceil_div(g.n0, k);
+    plane_forward<T, true>(a, st, jobs, nj, s0, FM_FAC_SQ, FM_FAC, 0);
+    for (int s = s0; s < s0 + nsteps; s++) {
+        xpass<T, 2>(a, st, jobs, nj, 0, 0, 1);
+        launch_after(any::ka_plane_mid<T>, dim3(mid_ctas, nj), plane_threads(a, mid_ctas * nj, km * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, km),
+                     st, g, jobs, 1, stack(g, km));
+        xpass<T, 1>(a, st, jobs, nj, 1, 1, 1);
+        if (s + 1 < s0 + nsteps)
+            launch_after(any::ka_plane_seam<T>, dim3(ctas, nj), plane_threads(a, ctas * nj, k * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, k), st,
+                         g, jobs, s, stack(g, k));
+        else
+            plane_inverse<T, true>(a, st, jobs, nj, s, 0, 0);
+    }
 }
 template <typename T> void step_discrete(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s, int half, int wf) {
     plane_forward<T, false>(a, st, jobs, nj, s, FM_NONE, 0, 0);
@@ -326,8 +343,8 @@ void any_destroy(AnyGrid *a) {
     if (a->tables) cudaFree(a->tables);
     delete a;
 }
-void any_step_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s) {
-    a->prec == 8 ? step_continuous<double>(a, st, jobs, nj, s) : step_continuous<float>(a, st, jobs, nj, s);
+void any_steps_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps) {
+    a->prec == 8 ? steps_continuous<double>(a, st, jobs, nj, s0, nsteps) : steps_continuous<float>(a, st, jobs, nj, s0, nsteps);
 }
 void any_step_discrete(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s, int half, int wf) {
     a->prec == 8 ? step_discrete<double>(a, st, jobs, nj, s, half, wf) : step_discrete<float>(a, st, jobs, nj, s, half, wf);
@@ -351,27 +368,38 @@ void any_xstress(const AnyGrid *a, cudaStream_t st, const lfts_step_job *sj, con
 // step in clusters of 16 against 27.7 (17.7 / 27.9); 256 points 16.2 / 25.4; 24^3 25 / 30;
 // 32^3, 32 768 points, 32.5 / 32.0 (26.6 / 30.4): the lines cross near 1500 (2500) points a
 // CTA.  More clusters than the device holds at once run in waves.
-int any_sweep_size(const AnyGrid *a, bool continuous, int nj, int force) {
-    const int *res = continuous ? a->clusters_cont : a->clusters_disc;
+int any_sweep_size(AnyGrid *a, bool continuous, int nj, int force) {
+    int *res = continuous ? a->clusters_cont : a->clusters_disc;
+    bool *asked = continuous ? a->asked_cont : a->asked_disc;
+    auto ask = [&](int k) {
+        if (res[k] && !asked[k]) {
+            asked[k] = true;
+            res[k] = a->prec == 8 ? (continuous ? resident_clusters(a, any::ka_sweep_continuous<double>, true, 1 << k)
+                                                : resident_clusters(a, any::ka_sweep_discrete<double>, false, 1 << k))
+                                  : (continuous ? resident_clusters(a, any::ka_sweep_continuous<float>, true, 1 << k)
+                                                : resident_clusters(a, any::ka_sweep_discrete<float>, false, 1 << k));
+        }
+        return res[k];
+    };
     if (force) {
         for (int k = 0; k < 5; k++)
-            if (1 << k == force && res[k]) return force;
+            if (1 << k == force && ask(k)) return force;
         return 0;
     }
     const bool f64 = a->prec == 8;
     const double M = (double)a->p.M, part = continuous ? 1.0 : 0.55;
     const double fixed = f64 ? 17.5 : 14.5, per_point = f64 ? 7.3e-3 : 4.8e-3;
     double best = part * (26.0 + nj * M * (f64 ? 5e-5 : 4e-5));
-    int size = 0;
+    int size = -1;
     for (int k = 0; k < 5; k++) {
         if (!res[k]) continue;
         const double t = part * ((nj + res[k] - 1) / res[k]) * (fixed + per_point * M / (1 << k));
         if (t < best) {
             best = t;
-            size = 1 << k;
+            size = k;
         }
     }
-    return size;
+    return size >= 0 && ask(size) ? 1 << size : 0;
 }
 int any_sweep_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps, int cs) {
     return a->prec == 8 ? sweep_continuous<double>(a, st, jobs, nj, s0, nsteps, cs) : sweep_continuous<float>(a, st, jobs, nj, s0, nsteps, cs);

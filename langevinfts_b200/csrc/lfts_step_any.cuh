@@ -281,6 +281,47 @@ __global__ void __launch_bounds__(NT_MAX) ka_plane_inverse(const __grid_constant
 }
 
 // ------------------------------------------------------------------------
+// The seam between two steps of a sweep: K5 of step s and K1 of step s + 1
+template <typename T>
+__global__ void __launch_bounds__(NT_MAX) ka_plane_seam(const __grid_constant__ Plan g, const lfts_step_job *__restrict__ jobs, int s,
+                                                        Stack sk) {
+    using C = typename CT<T>::type;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    PlaneBuf<C> sm(smem_raw, g, sk.planes);
+    const lfts_step_job jb = jobs[blockIdx.y];
+    grid_wait();
+    if (jb.active && !jb.active[jb.replica]) return;
+    const int x0 = blockIdx.x * sk.planes, np = min(sk.planes, g.n0 - x0), area = g.n1 * g.n2, half = g.n1 * g.nzc;
+    C *spec = (C *)jb.spec + (size_t)x0 * half;
+    load_packed<C, true>(g, spec, sm.buf, np, np);
+    __syncthreads();
+    plane_inverse(g, sm.buf, sk, sm.twy, sm.twz);
+    const T *fac = (const T *)jb.fac + (long long)x0 * area;
+    T *qout = (T *)jb.out + s * jb.out_stride + (long long)x0 * area;
+    for (int i = threadIdx.x; i < np * area; i += blockDim.x) {
+        const Point pt = point_at(g, i, sm.iy, sm.iz);
+        const int src = (pt.p * g.n1 + pt.y) * g.n2 + pt.t;
+        const T eh = fac[src];
+        C z = sm.buf[pt.o];
+        const T q = third((T)4 * eh * z.y - eh * eh * z.x);
+        qout[src] = q;
+        z.x = q * (eh * eh);
+        z.y = q * eh;
+        sm.buf[pt.o] = z;
+    }
+    __syncthreads();
+    plane_forward(g, sm.buf, sk, sm.twy, sm.twz);
+    for (int i = threadIdx.x; i < np * half; i += blockDim.x) {
+        const int r = fdiv(i, g.mul_nzc), kz = i - r * g.nzc;
+        const int p = fdiv(r, g.mul_n1), ky = r - p * g.n1;
+        C A, B;
+        separate(sm.buf[r * g.pitch + kz], sm.buf[(p * g.n1 + (ky ? g.n1 - ky : 0)) * g.pitch + (kz ? g.n2 - kz : 0)], A, B);
+        spec[i] = A;
+        spec[g.Mc + i] = B;
+    }
+}
+
+// ------------------------------------------------------------------------
 // Tiles of TJ (y, kz) columns, NBR spectra side by side: rows x, NBR * TJ wide
 template <typename C>
 struct TileBuf {

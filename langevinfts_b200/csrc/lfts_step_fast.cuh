@@ -493,5 +493,98 @@ __global__ void __launch_bounds__(NT) kf_plane_inverse(GridPlan g, const lfts_st
     }
 }
 
+// ------------------------------------------------------------------------
+// The seam between two steps of a sweep: K5 of step s and K1 of step s + 1 on one
+// plane.  A warp keeps q' of its rows in registers between the two z transforms.
+template <typename T, int N, int NT = NTHR>
+__global__ void __launch_bounds__(NT) kf_plane_seam(GridPlan g, const lfts_step_job *__restrict__ jobs, int s) {
+    using C = typename CT<T>::type;
+    using SM = FSmem<C, N, 2, 1, NT>;
+    constexpr int NZC = SM::NZC, PL = SM::PL, ZB = SM::ZB, PER = (N + 31) / 32;
+    using LZ = Lines<ZB, 1, PL, 1, true, false>;
+    using LY = Lines<2 * NZC, NZC, N * NZC, NZC, false, true>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C *P = (C *)smem_raw;
+    C *zl = P + SM::P_ELEMS;
+    C *stw = zl + SM::Z_ELEMS;
+    const lfts_step_job jb = jobs[blockIdx.y];
+    load_stw<C, N, NT>(stw, g.stw);
+    grid_wait();
+    if (jb.active && !jb.active[jb.replica]) return;
+    const int x = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __syncthreads();
+    fload_inverse_y<C, N, 2, NT>(g, jb, 0, P, stw);
+    const long long poff = (long long)x * N * N;
+    const T *fac = (const T *)jb.fac + poff;
+    T *qout = (T *)jb.out + s * jb.out_stride + poff;
+    C *zw = zl + warp * ZB * PL;
+    for (int u0 = warp * ZB; u0 < N; u0 += (NT / 32) * ZB) {
+        T fa[ZB][PER];
+#pragma unroll
+        for (int b = 0; b < ZB; b++) {
+#pragma unroll
+            for (int i = 0; i < PER; i++) {
+                const int t = lane + 32 * i;
+                if (u0 + b < N && t < N) fa[b][i] = fac[(u0 + b) * N + t];
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < ZB; b++) {
+            if (u0 + b >= N) break;
+            const C *rowA = P + perm_ct<N>(u0 + b) * NZC, *rowB = rowA + N * NZC;
+            for (int k = lane; k < N; k += 32) zw[b * PL + LZ::off(perm_ct<N>(k))] = pack_pair(rowA, rowB, k, N, NZC);
+        }
+        __syncwarp();
+        dit<LZ, N, false>(zw, stw, +1, lane, 32);
+        C v[ZB][PER];
+#pragma unroll
+        for (int b = 0; b < ZB; b++) {
+#pragma unroll
+            for (int i = 0; i < PER; i++) {
+                const int t = lane + 32 * i;
+                if (u0 + b < N && t < N) {
+                    const C z = zw[b * PL + LZ::off(t)];
+                    const T eh = fa[b][i], q = ((T)4 * eh * z.y - eh * eh * z.x) / (T)3;
+                    qout[(u0 + b) * N + t] = q;
+                    v[b][i].x = q * (eh * eh);
+                    v[b][i].y = q * eh;
+                }
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int b = 0; b < ZB; b++) {
+#pragma unroll
+            for (int i = 0; i < PER; i++) {
+                const int t = lane + 32 * i;
+                if (u0 + b < N && t < N) zw[b * PL + LZ::off(perm_ct<N>(t))] = v[b][i];
+            }
+        }
+        __syncwarp();
+        dit<LZ, N, false>(zw, stw, -1, lane, 32);
+#pragma unroll
+        for (int b = 0; b < ZB; b++) {
+            if (u0 + b >= N) break;
+            C *rowA = P + perm_ct<N>(u0 + b) * NZC, *rowB = rowA + N * NZC;
+            const C *z = zw + b * PL;
+            for (int k = lane; k < NZC; k += 32) {
+                C A, B;
+                split_pair(z[LZ::off(k)], cconj(z[LZ::off(k == 0 ? 0 : N - k)]), A, B);
+                rowA[k] = A;
+                rowB[k] = B;
+            }
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    dit<LY, N, true>(P, stw, -1, tid, NT);
+#pragma unroll
+    for (int b = 0; b < 2; b++) {
+        C *out = (C *)jb.spec + (size_t)b * g.Mc + (size_t)x * N * NZC;
+        const C *src = P + b * N * NZC;
+        for (int i = tid; i < N * NZC; i += NT) out[i] = src[i];
+    }
+}
+
 }  // namespace fast
 }  // namespace lfts

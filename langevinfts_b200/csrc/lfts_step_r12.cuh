@@ -254,6 +254,69 @@ __device__ __forceinline__ void put_packed(C *P, int y, int kz, int kc, C A, C B
 template <typename T> __host__ __device__ constexpr int minb_two_branch() { return sizeof(T) == 4 ? 2 : 1; }
 template <typename T> __host__ __device__ constexpr int minb_mid() { return sizeof(T) == 4 ? 2 : 1; }
 
+// The y half of K1: columns of the packed plane split into the spectra of both branches
+template <typename C>
+__device__ __forceinline__ void split_columns_forward(C *P, C *out, long long Mc, int grp, int j, C wf, unsigned mask) {
+    // y-columns: task kz splits columns kz and kc into the branches; branch 1
+    // waits in column kc while branch 0 is transformed and stored
+    const int kz = grp, kc = kz == 0 ? N / 2 : N - kz;
+    C A[12];
+#pragma unroll
+    for (int m = 0; m < 12; m++) {
+        const int y = j + 8 * m;
+        const C zk = P[at<C>(y, kz)], zc = P[at<C>(y, kc)];
+        C b;
+        if (kz != 0) {
+            split_pair(zk, cconj(zc), A[m], b);
+        } else {
+            A[m].x = zk.x;  // branch 0: DC + i Nyquist
+            A[m].y = zc.x;
+            b.x = zk.y;  // branch 1
+            b.y = zc.y;
+        }
+        P[at<C>(y, kc)] = b;
+    }
+    __syncwarp(mask);
+    C o0[8], o1[8];
+    fft96a<-1>(A, Col<C>{P, kz}, j, wf, mask, o0, o1);
+    put_columns(out, Col<C>{P, kz}, kz, o0, o1, j, mask);
+#pragma unroll
+    for (int m = 0; m < 12; m++) A[m] = P[at<C>(j + 8 * m, kc)];
+    __syncwarp(mask);
+    fft96a<-1>(A, Col<C>{P, kc}, j, wf, mask, o0, o1);
+    put_columns(out + Mc, Col<C>{P, kc}, kz, o0, o1, j, mask);
+}
+// The y half of K5: spectra of both branches joined into the columns of the packed plane
+template <typename C>
+__device__ __forceinline__ void join_columns_inverse(C *P, const C *in, long long Mc, int grp, int j, C wi, unsigned mask) {
+    // branch 0 waits in column kz (rows y) while branch 1 is transformed,
+    // then both are packed into the z-lines
+    const int kz = grp, kc = kz == 0 ? N / 2 : N - kz;
+    C A[12], o0[8], o1[8];
+    get_columns(in, kz, A, j);
+    fft96a<+1>(A, Col<C>{P, kz}, j, wi, mask, o0, o1);
+#pragma unroll
+    for (int k = 0; k < 8; k++) P[at<C>(j + 12 * k, kz)] = o0[k];
+    if (j < 4) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) P[at<C>(8 + j + 12 * k, kz)] = o1[k];
+    }
+    get_columns(in + Mc, kz, A, j);
+    fft96a<+1>(A, Col<C>{P, kc}, j, wi, mask, o0, o1);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int y = j + 12 * k;
+        put_packed(P, y, kz, kc, P[at<C>(y, kz)], o0[k]);
+    }
+    if (j < 4) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const int y = 8 + j + 12 * k;
+            put_packed(P, y, kz, kc, P[at<C>(y, kz)], o1[k]);
+        }
+    }
+}
+
 // ------------------------------------------------------------------------
 // K1: forward zy transform of one x-plane into the spectra of f0(fac) q and
 // f1(fac) q (slots spec_out0, spec_out0 + 1).
@@ -301,34 +364,7 @@ __global__ void __launch_bounds__(NT, minb_two_branch<T>()) kq_plane_forward(Gri
         }
     }
     __syncthreads();
-    // y-columns: task kz splits columns kz and kc into the branches; branch 1
-    // waits in column kc while branch 0 is transformed and stored
-    const int kz = grp, kc = kz == 0 ? N / 2 : N - kz;
-    C A[12];
-#pragma unroll
-    for (int m = 0; m < 12; m++) {
-        const int y = j + 8 * m;
-        const C zk = P[at<C>(y, kz)], zc = P[at<C>(y, kc)];
-        C b;
-        if (kz != 0) {
-            split_pair(zk, cconj(zc), A[m], b);
-        } else {
-            A[m].x = zk.x;  // branch 0: DC + i Nyquist
-            A[m].y = zc.x;
-            b.x = zk.y;  // branch 1
-            b.y = zc.y;
-        }
-        P[at<C>(y, kc)] = b;
-    }
-    __syncwarp(mask);
-    C o0[8], o1[8];
-    fft96a<-1>(A, Col<C>{P, kz}, j, wf, mask, o0, o1);
-    put_columns(out, Col<C>{P, kz}, kz, o0, o1, j, mask);
-#pragma unroll
-    for (int m = 0; m < 12; m++) A[m] = P[at<C>(j + 8 * m, kc)];
-    __syncwarp(mask);
-    fft96a<-1>(A, Col<C>{P, kc}, j, wf, mask, o0, o1);
-    put_columns(out + g.Mc, Col<C>{P, kc}, kz, o0, o1, j, mask);
+    split_columns_forward(P, out, g.Mc, grp, j, wf, mask);
 }
 
 // ------------------------------------------------------------------------
@@ -440,34 +476,7 @@ __global__ void __launch_bounds__(NT, minb_two_branch<T>()) kq_plane_inverse(Gri
     const T *fac = (const T *)jb.fac + poff;
     T *qout = (T *)jb.out + s * jb.out_stride + poff;
     const T THIRD = (T)(1.0 / 3.0);
-    {
-        // branch 0 waits in column kz (rows y) while branch 1 is transformed,
-        // then both are packed into the z-lines
-        const int kz = grp, kc = kz == 0 ? N / 2 : N - kz;
-        C A[12], o0[8], o1[8];
-        get_columns(in, kz, A, j);
-        fft96a<+1>(A, Col<C>{P, kz}, j, wi, mask, o0, o1);
-#pragma unroll
-        for (int k = 0; k < 8; k++) P[at<C>(j + 12 * k, kz)] = o0[k];
-        if (j < 4) {
-#pragma unroll
-            for (int k = 0; k < 8; k++) P[at<C>(8 + j + 12 * k, kz)] = o1[k];
-        }
-        get_columns(in + g.Mc, kz, A, j);
-        fft96a<+1>(A, Col<C>{P, kc}, j, wi, mask, o0, o1);
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int y = j + 12 * k;
-            put_packed(P, y, kz, kc, P[at<C>(y, kz)], o0[k]);
-        }
-        if (j < 4) {
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const int y = 8 + j + 12 * k;
-                put_packed(P, y, kz, kc, P[at<C>(y, kz)], o1[k]);
-            }
-        }
-    }
+    join_columns_inverse(P, in, g.Mc, grp, j, wi, mask);
     __syncthreads();
     for (int y = grp; y < N; y += GROUPS) {
         const T *frow = fac + y * N;
@@ -491,6 +500,68 @@ __global__ void __launch_bounds__(NT, minb_two_branch<T>()) kq_plane_inverse(Gri
             for (int k = 0; k < 8; k++) qrow[8 + j + 12 * k] = ((T)4 * e1[k] * o1[k].y - e1[k] * e1[k] * o1[k].x) * THIRD;
         }
     }
+}
+
+// ------------------------------------------------------------------------
+// The seam between two steps of a sweep: K5 of step s and K1 of step s + 1 on one
+// plane (see lfts_step_r8.cuh).  The inverse line ends in variant A's distribution,
+// from which variant B transforms forward with no further exchange.
+template <typename T>
+__global__ void __launch_bounds__(NT, minb_two_branch<T>()) kq_plane_seam(GridPlan g, const lfts_step_job *__restrict__ jobs, int s) {
+    using C = typename CT<T>::type;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C *P = (C *)smem_raw;
+    const lfts_step_job jb = jobs[blockIdx.y];
+    const int x = blockIdx.x, tid = threadIdx.x, lane = tid & 31, j = lane & 7, grp = tid >> 3;
+    const unsigned mask = 0xFFu << (lane & 24);
+    const C wi = tw96<C>(j, +1), wf = tw96<C>(j, -1), wf8 = tw96<C>(8 + j, -1);
+    grid_wait();
+    if (jb.active && !jb.active[jb.replica]) return;
+    C *sp = (C *)jb.spec + (size_t)x * PLANE;
+    const long long poff = (long long)x * N * N;
+    const T *fac = (const T *)jb.fac + poff;
+    T *qout = (T *)jb.out + s * jb.out_stride + poff;
+    const T THIRD = (T)(1.0 / 3.0);
+    join_columns_inverse(P, (const C *)sp, g.Mc, grp, j, wi, mask);
+    __syncthreads();
+    for (int y = grp; y < N; y += GROUPS) {
+        const T *frow = fac + y * N;
+        T *qrow = qout + y * N;
+        T e0[8], e1[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) e0[k] = frow[j + 12 * k];
+        if (j < 4) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) e1[k] = frow[8 + j + 12 * k];
+        }
+        C a[12], o0[8], o1[8];
+#pragma unroll
+        for (int m = 0; m < 12; m++) a[m] = P[at<C>(y, j + 8 * m)];
+        __syncwarp(mask);
+        fft96a<+1>(a, Row<C>{P, y}, j, wi, mask, o0, o1);
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const T q = ((T)4 * e0[k] * o0[k].y - e0[k] * e0[k] * o0[k].x) * THIRD;
+            qrow[j + 12 * k] = q;
+            o0[k].x = q * (e0[k] * e0[k]);
+            o0[k].y = q * e0[k];
+        }
+        if (j < 4) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const T q = ((T)4 * e1[k] * o1[k].y - e1[k] * e1[k] * o1[k].x) * THIRD;
+                qrow[8 + j + 12 * k] = q;
+                o1[k].x = q * (e1[k] * e1[k]);
+                o1[k].y = q * e1[k];
+            }
+        }
+        __syncwarp(mask);
+        fft96b<-1>(o0, o1, Row<C>{P, y}, j, wf, wf8, mask, a);
+#pragma unroll
+        for (int k = 0; k < 12; k++) P[at<C>(y, j + 8 * k)] = a[k];
+    }
+    __syncthreads();
+    split_columns_forward(P, sp, g.Mc, grp, j, wf, mask);
 }
 
 // ------------------------------------------------------------------------

@@ -261,6 +261,74 @@ __device__ __forceinline__ void y_inverse_paired(C *P, int kz, int j, C wi, unsi
     put_zlines_paired<C>(P, kz, j, a);
 }
 
+// The y half of K1: columns of the packed plane split into the spectra of both branches
+template <typename C>
+__device__ __forceinline__ void split_columns_forward(C *P, C *out, long long Mc, int grp, int j, int lane, C wf, unsigned mask) {
+    // y-columns: task kz splits the branches; branch 1 waits in its own
+    // column (ekc) while branch 0 is transformed and stored
+    const int kz = grp, ekz = kz, ekc = kz == 0 ? N / 2 : N - kz;
+    C A[8];
+#pragma unroll
+    for (int m = 0; m < 8; m++) {
+        const int y = j + 8 * m;
+        const C zk = P[at<C>(y, ekz)], zc = P[at<C>(y, ekc)];
+        C b;
+        if (kz != 0) {
+            split_pair(zk, cconj(zc), A[m], b);
+        } else {
+            A[m].x = zk.x;  // branch 0: DC + i Nyquist
+            A[m].y = zc.x;
+            b.x = zk.y;  // branch 1
+            b.y = zc.y;
+        }
+        P[at<C>(y, ekc)] = b;
+    }
+    __syncwarp(mask);
+    fft64<-1>(A, ColS<C>{P, ekz}, j, wf, mask);
+    put_columns(out, kz, A, j, lane, mask);
+#pragma unroll
+    for (int m = 0; m < 8; m++) A[m] = P[at<C>(j + 8 * m, ekc)];
+    __syncwarp(mask);
+    fft64<-1>(A, ColS<C>{P, ekc}, j, wf, mask);
+    put_columns(out + Mc, kz, A, j, lane, mask);
+}
+// The y half of K5: spectra of both branches joined into the columns of the packed plane
+template <typename C>
+__device__ __forceinline__ void join_columns_inverse(C *P, const C *in, long long Mc, int grp, int j, C wi, unsigned mask) {
+    // branch 0 first; its inverse column waits in column ekz while
+    // branch 1 is transformed, then both are packed into the z-lines
+    const int kz = grp, ekz = kz, ekc = kz == 0 ? N / 2 : N - kz;
+    C A[8];
+    get_columns(in, kz, A, j);
+    fft64<+1>(A, ColS<C>{P, ekz}, j, wi, mask);
+#pragma unroll
+    for (int k = 0; k < 8; k++) P[at<C>(j + 8 * k, ekz)] = A[k];
+    get_columns(in + Mc, kz, A, j);
+    fft64<+1>(A, ColS<C>{P, ekc}, j, wi, mask);
+    // z-line y = j + 8k: A + i B (Hermitian extension at 64 - kz)
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int y = j + 8 * k;
+        const C a = P[at<C>(y, ekz)], bb = A[k];
+        C z;
+        if (kz != 0) {
+            z.x = a.x - bb.y;
+            z.y = a.y + bb.x;
+            P[at<C>(y, ekz)] = z;
+            z.x = a.x + bb.y;
+            z.y = -a.y + bb.x;
+            P[at<C>(y, ekc)] = z;
+        } else {
+            z.x = a.x;  // A(kz = 0) + i B(kz = 0)
+            z.y = bb.x;
+            P[at<C>(y, ekz)] = z;
+            z.x = a.y;  // A(kz = 32) + i B(kz = 32)
+            z.y = bb.y;
+            P[at<C>(y, ekc)] = z;
+        }
+    }
+}
+
 // ------------------------------------------------------------------------
 // K1: forward zy transform of one x-plane.
 //   NBR = 2: spectra of f0(fac) q and f1(fac) q (slots spec_out0, +1);
@@ -307,33 +375,7 @@ __global__ void __launch_bounds__(NTHR, (sizeof(T) == 4 ? LFTS_R8_MINB_F32 : LFT
             for (int k = 0; k < 8; k++) P[at<C>(y, 8 * k + j)] = a[k];
         }
         __syncthreads();
-        // y-columns: task kz splits the branches; branch 1 waits in its own
-        // column (ekc) while branch 0 is transformed and stored
-        const int kz = grp, ekz = kz, ekc = kz == 0 ? N / 2 : N - kz;
-        C A[8];
-#pragma unroll
-        for (int m = 0; m < 8; m++) {
-            const int y = j + 8 * m;
-            const C zk = P[at<C>(y, ekz)], zc = P[at<C>(y, ekc)];
-            C b;
-            if (kz != 0) {
-                split_pair(zk, cconj(zc), A[m], b);
-            } else {
-                A[m].x = zk.x;  // branch 0: DC + i Nyquist
-                A[m].y = zc.x;
-                b.x = zk.y;  // branch 1
-                b.y = zc.y;
-            }
-            P[at<C>(y, ekc)] = b;
-        }
-        __syncwarp(mask);
-        fft64<-1>(A, ColS<C>{P, ekz}, j, wf, mask);
-        put_columns(out, kz, A, j, lane, mask);
-#pragma unroll
-        for (int m = 0; m < 8; m++) A[m] = P[at<C>(j + 8 * m, ekc)];
-        __syncwarp(mask);
-        fft64<-1>(A, ColS<C>{P, ekc}, j, wf, mask);
-        put_columns(out + g.Mc, kz, A, j, lane, mask);
+        split_columns_forward(P, out, g.Mc, grp, j, lane, wf, mask);
     } else {
         // z-lines: rows u and u + 32 packed as real / imaginary part
         {
@@ -568,40 +610,7 @@ __global__ void __launch_bounds__(NTHR, (sizeof(T) == 4 ? LFTS_R8_MINB_F32 : LFT
     T *qout = (T *)jb.out + s * jb.out_stride + poff;
     const T THIRD = (T)(1.0 / 3.0);  // multiply, not divide: no iterative division per element
     if (NBR == 2) {
-        {
-            // branch 0 first; its inverse column waits in column ekz while
-            // branch 1 is transformed, then both are packed into the z-lines
-            const int kz = grp, ekz = kz, ekc = kz == 0 ? N / 2 : N - kz;
-            C A[8];
-            get_columns(in, kz, A, j);
-            fft64<+1>(A, ColS<C>{P, ekz}, j, wi, mask);
-#pragma unroll
-            for (int k = 0; k < 8; k++) P[at<C>(j + 8 * k, ekz)] = A[k];
-            get_columns(in + g.Mc, kz, A, j);
-            fft64<+1>(A, ColS<C>{P, ekc}, j, wi, mask);
-            // z-line y = j + 8k: A + i B (Hermitian extension at 64 - kz)
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const int y = j + 8 * k;
-                const C a = P[at<C>(y, ekz)], bb = A[k];
-                C z;
-                if (kz != 0) {
-                    z.x = a.x - bb.y;
-                    z.y = a.y + bb.x;
-                    P[at<C>(y, ekz)] = z;
-                    z.x = a.x + bb.y;
-                    z.y = -a.y + bb.x;
-                    P[at<C>(y, ekc)] = z;
-                } else {
-                    z.x = a.x;  // A(kz = 0) + i B(kz = 0)
-                    z.y = bb.x;
-                    P[at<C>(y, ekz)] = z;
-                    z.x = a.y;  // A(kz = 32) + i B(kz = 32)
-                    z.y = bb.y;
-                    P[at<C>(y, ekc)] = z;
-                }
-            }
-        }
+        join_columns_inverse(P, in, g.Mc, grp, j, wi, mask);
         __syncthreads();
         for (int y = grp; y < N; y += GROUPS) {
             const T *frow = fac + y * N + j;
@@ -638,6 +647,56 @@ __global__ void __launch_bounds__(NTHR, (sizeof(T) == 4 ? LFTS_R8_MINB_F32 : LFT
             qout[(u + 32) * N + j + 8 * k] = a[k].y * fmul_mode(fm0, fb[k]);
         }
     }
+}
+
+// ------------------------------------------------------------------------
+// The seam between two steps of a sweep: K5 of step s and K1 of step s + 1 on one
+// plane.  A z-line's lane holds q' of exactly the elements the forward transform
+// starts from, so q' goes to memory and on, in registers, into the next step: one
+// launch, a pass over q and one over fac less a step.
+template <typename T>
+__global__ void __launch_bounds__(NTHR, (sizeof(T) == 4 ? LFTS_R8_MINB_F32 : LFTS_R8_MINB)) kr_plane_seam(GridPlan g, const lfts_step_job *__restrict__ jobs, int s) {
+    using C = typename CT<T>::type;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C *P = (C *)smem_raw;
+    const lfts_step_job jb = jobs[blockIdx.y];
+    const int x = blockIdx.x, tid = threadIdx.x, lane = tid & 31, j = lane & 7, grp = tid >> 3;
+    const unsigned mask = 0xFFu << (lane & 24);
+    const C wi = tw_base<C>(j, +1), wf = tw_base<C>(j, -1);
+    grid_wait();
+    if (jb.active && !jb.active[jb.replica]) return;
+    C *sp = (C *)jb.spec + (size_t)x * PLANE;
+    const long long poff = (long long)x * N * N;
+    const T *fac = (const T *)jb.fac + poff;
+    T *qout = (T *)jb.out + s * jb.out_stride + poff;
+    const T THIRD = (T)(1.0 / 3.0);
+    join_columns_inverse(P, (const C *)sp, g.Mc, grp, j, wi, mask);
+    __syncthreads();
+    for (int y = grp; y < N; y += GROUPS) {
+        const T *frow = fac + y * N + j;
+        T *qrow = qout + y * N + j;
+        T eh[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) eh[k] = frow[8 * k];
+        C a[8];
+#pragma unroll
+        for (int m = 0; m < 8; m++) a[m] = P[at<C>(y, 8 * m + j)];
+        __syncwarp(mask);
+        fft64<+1>(a, RowX<C>{P, y}, j, wi, mask);
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const T q = ((T)4 * eh[k] * a[k].y - eh[k] * eh[k] * a[k].x) * THIRD;
+            qrow[8 * k] = q;
+            a[k].x = q * (eh[k] * eh[k]);
+            a[k].y = q * eh[k];
+        }
+        __syncwarp(mask);
+        fft64<-1>(a, RowX<C>{P, y}, j, wf, mask);
+#pragma unroll
+        for (int k = 0; k < 8; k++) P[at<C>(y, 8 * k + j)] = a[k];
+    }
+    __syncthreads();
+    split_columns_forward(P, sp, g.Mc, grp, j, lane, wf, mask);
 }
 
 }  // namespace r8
