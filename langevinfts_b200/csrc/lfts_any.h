@@ -16,7 +16,7 @@ AnyGrid *any_create(int prec, const int n[3], int nsm, int max_smem, std::string
 void any_destroy(AnyGrid *a);
 
 void any_steps_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps);
-void any_step_discrete(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s, int half, int with_fac);
+void any_steps_discrete(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps, int half, int with_fac);
 // zy-transforms of one real field per job into spectrum slot 0 (half the 3D transform)
 void any_planes_forward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj);
 void any_xpass_forward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj);

@@ -157,6 +157,7 @@ template <typename T, int N> static int fast_setup(int max_smem) {
     if (allow_smem(fast::kf_plane_forward<T, 1, N>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(fast::kf_plane_forward<T, 2, N, NT2>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(fast::kf_plane_mid<T, N>, max_smem) != cudaSuccess) return 0;
+    if (allow_smem(fast::kf_plane_mid<T, N, NTHR, true>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(fast::kf_plane_inverse<T, 2, EPI_RICH, N, NT2>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(fast::kf_plane_inverse<T, 1, EPI_SCALE, N>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(fast::kf_plane_seam<T, N, NT2>, max_smem) != cudaSuccess) return 0;
@@ -186,6 +187,7 @@ template <typename T> static int r8_setup(int max_smem) {
     if (allow_smem(r8::kr_plane_forward<T, 1, FM_NONE, FM_NONE>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(r8::kr_plane_forward<T, 2, FM_FAC_SQ, FM_FAC>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(r8::kr_plane_mid<T>, max_smem) != cudaSuccess) return 0;
+    if (allow_smem(r8::kr_plane_mid<T, true>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(r8::kr_plane_inverse<T, 2, EPI_RICH>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(r8::kr_plane_inverse<T, 1, EPI_SCALE>, max_smem) != cudaSuccess) return 0;
     if (allow_smem(r8::kr_plane_seam<T>, max_smem) != cudaSuccess) return 0;
@@ -642,7 +644,7 @@ static int steps_cont_fast(lfts_ctx c, const lfts_step_job *jobs, int nj, int s0
             CK(launch_after(r8::kr_plane_forward<T, 2, FM_FAC_SQ, FM_FAC>, dim3(rp), NTHR, ps, st, g, jobs, s0, 0));
             for (int s = s0; s <= last; s++) {
                 CK(launch_after(r8::kp_xpass<T, 2>, dim3(px2), NTHR, r8::xpipe_smem<C>(), st, g, jobs, nj, 0, 0, 1));
-                CK(launch_after(r8::kr_plane_mid<T>, dim3(rp), NTHR, ps, st, g, jobs, 1));
+                CK(launch_after(r8::kr_plane_mid<T>, dim3(rp), NTHR, ps, st, g, jobs, 1, 0));
                 CK(launch_after(r8::kp_xpass<T, 1>, dim3(px1), NTHR, r8::xpipe_smem<C>(), st, g, jobs, nj, 1, 1, 1));
                 if (s < last) CK(launch_after(r8::kr_plane_seam<T>, dim3(rp), NTHR, ps, st, g, jobs, s));
                 else CK(launch_after(r8::kr_plane_inverse<T, 2, EPI_RICH>, dim3(rp), NTHR, ps, st, g, jobs, s, 0, 0));
@@ -678,7 +680,7 @@ static int steps_cont_fast(lfts_ctx c, const lfts_step_job *jobs, int nj, int s0
     CK(launch_after(fast::kf_plane_forward<T, 2, N, NT2>, dim3(gp), NT2, f2, st, g, jobs, s0, FM_FAC_SQ, FM_FAC, 0));
     for (int s = s0; s <= last; s++) {
         CK(launch_after(fast::kf_xpass<T, 2, N>, dim3(gx), NTHR, x2, st, g, jobs, 0, 0, 1));
-        CK(launch_after(fast::kf_plane_mid<T, N>, dim3(gp), NTHR, f1, st, g, jobs, 1));
+        CK(launch_after(fast::kf_plane_mid<T, N>, dim3(gp), NTHR, f1, st, g, jobs, 1, 0));
         CK(launch_after(fast::kf_xpass<T, 1, N>, dim3(gx), NTHR, x1, st, g, jobs, 1, 1, 1));
         if (s < last) CK(launch_after(fast::kf_plane_seam<T, N, NT2>, dim3(gp), NT2, f2, st, g, jobs, s));
         else CK(launch_after(fast::kf_plane_inverse<T, 2, EPI_RICH, N, NT2>, dim3(gp), NT2, f2, st, g, jobs, s, 0, 0));
@@ -686,11 +688,13 @@ static int steps_cont_fast(lfts_ctx c, const lfts_step_job *jobs, int nj, int s0
     CKLAUNCH();
     return 0;
 }
+// K1, then per step K2 and the seam to the next (with_fac), K5 after the last
 template <typename T, int N>
-static int step_disc_fast(lfts_ctx c, const lfts_step_job *jobs, int nj, int s, int half, int with_fac) {
+static int steps_disc_fast(lfts_ctx c, const lfts_step_job *jobs, int nj, int s0, int nsteps, int half, int with_fac) {
     using C = typename CT<T>::type;
     const GridPlan &g = c->g;
     cudaStream_t st = c->stream;
+    const int last = s0 + nsteps - 1;
     constexpr int TJ = sizeof(T) == 8 ? 16 : 32;
     const dim3 gp(N, nj), gx((unsigned)(((long long)N * (N / 2 + 1) + TJ - 1) / TJ), nj);
     const size_t f1 = fast::FSmem<C, N, 1, 1>::BYTES;
@@ -699,29 +703,35 @@ static int step_disc_fast(lfts_ctx c, const lfts_step_job *jobs, int nj, int s, 
         if (c->r8) {
             const dim3 rp(N, nj);
             const size_t ps = r8::plane_smem<C>();
-            CK(launch_after(r8::kr_plane_forward<T, 1, FM_NONE, FM_NONE>, dim3(rp), NTHR, ps, st, g, jobs, s, 0));
+            CK(launch_after(r8::kr_plane_forward<T, 1, FM_NONE, FM_NONE>, dim3(rp), NTHR, ps, st, g, jobs, s0, 0));
             const long long it1 = (long long)nj * r8::xpipe_tiles<C>(), cap = (long long)(c->xcap ? c->xcap : 3) * c->nsm;
-            CK(launch_after(r8::kp_xpass<T, 1>, dim3((unsigned)(it1 < cap ? it1 : cap)), NTHR, r8::xpipe_smem<C>(), st, g, jobs, nj, 0, half, half));
-            CK(launch_after(r8::kr_plane_inverse<T, 1, EPI_SCALE>, dim3(rp), NTHR, ps, st, g, jobs, s, 0, with_fac ? FM_FAC : FM_NONE));
+            for (int s = s0; s <= last; s++) {
+                CK(launch_after(r8::kp_xpass<T, 1>, dim3((unsigned)(it1 < cap ? it1 : cap)), NTHR, r8::xpipe_smem<C>(), st, g, jobs, nj, 0, half, half));
+                if (s < last) CK(launch_after(r8::kr_plane_mid<T, true>, dim3(rp), NTHR, ps, st, g, jobs, 0, s));
+                else CK(launch_after(r8::kr_plane_inverse<T, 1, EPI_SCALE>, dim3(rp), NTHR, ps, st, g, jobs, s, 0, with_fac ? FM_FAC : FM_NONE));
+            }
             CKLAUNCH();
             return 0;
         }
     }
-    CK(launch_after(fast::kf_plane_forward<T, 1, N>, dim3(gp), NTHR, f1, st, g, jobs, s, FM_NONE, 0, 0));
-    CK(launch_after(fast::kf_xpass<T, 1, N>, dim3(gx), NTHR, x1, st, g, jobs, 0, half, half));
-    CK(launch_after(fast::kf_plane_inverse<T, 1, EPI_SCALE, N>, dim3(gp), NTHR, f1, st, g, jobs, s, 0, with_fac ? FM_FAC : FM_NONE));
+    CK(launch_after(fast::kf_plane_forward<T, 1, N>, dim3(gp), NTHR, f1, st, g, jobs, s0, FM_NONE, 0, 0));
+    for (int s = s0; s <= last; s++) {
+        CK(launch_after(fast::kf_xpass<T, 1, N>, dim3(gx), NTHR, x1, st, g, jobs, 0, half, half));
+        if (s < last) CK(launch_after(fast::kf_plane_mid<T, N, NTHR, true>, dim3(gp), NTHR, f1, st, g, jobs, 0, s));
+        else CK(launch_after(fast::kf_plane_inverse<T, 1, EPI_SCALE, N>, dim3(gp), NTHR, f1, st, g, jobs, s, 0, with_fac ? FM_FAC : FM_NONE));
+    }
     CKLAUNCH();
     return 0;
 }
 template <typename T>
 static int step_fast_dispatch(lfts_ctx c, const lfts_step_job *jobs, int nj, int s, int nsteps, int disc, int half, int wf) {
     switch (c->fastN) {
-        case 16: return disc ? step_disc_fast<T, 16>(c, jobs, nj, s, half, wf) : steps_cont_fast<T, 16>(c, jobs, nj, s, nsteps);
-        case 32: return disc ? step_disc_fast<T, 32>(c, jobs, nj, s, half, wf) : steps_cont_fast<T, 32>(c, jobs, nj, s, nsteps);
-        case 48: return disc ? step_disc_fast<T, 48>(c, jobs, nj, s, half, wf) : steps_cont_fast<T, 48>(c, jobs, nj, s, nsteps);
-        case 64: return disc ? step_disc_fast<T, 64>(c, jobs, nj, s, half, wf) : steps_cont_fast<T, 64>(c, jobs, nj, s, nsteps);
-        case 96: return disc ? step_disc_fast<T, 96>(c, jobs, nj, s, half, wf) : steps_cont_fast<T, 96>(c, jobs, nj, s, nsteps);
-        case 128: return disc ? step_disc_fast<T, 128>(c, jobs, nj, s, half, wf) : steps_cont_fast<T, 128>(c, jobs, nj, s, nsteps);
+        case 16: return disc ? steps_disc_fast<T, 16>(c, jobs, nj, s, nsteps, half, wf) : steps_cont_fast<T, 16>(c, jobs, nj, s, nsteps);
+        case 32: return disc ? steps_disc_fast<T, 32>(c, jobs, nj, s, nsteps, half, wf) : steps_cont_fast<T, 32>(c, jobs, nj, s, nsteps);
+        case 48: return disc ? steps_disc_fast<T, 48>(c, jobs, nj, s, nsteps, half, wf) : steps_cont_fast<T, 48>(c, jobs, nj, s, nsteps);
+        case 64: return disc ? steps_disc_fast<T, 64>(c, jobs, nj, s, nsteps, half, wf) : steps_cont_fast<T, 64>(c, jobs, nj, s, nsteps);
+        case 96: return disc ? steps_disc_fast<T, 96>(c, jobs, nj, s, nsteps, half, wf) : steps_cont_fast<T, 96>(c, jobs, nj, s, nsteps);
+        case 128: return disc ? steps_disc_fast<T, 128>(c, jobs, nj, s, nsteps, half, wf) : steps_cont_fast<T, 128>(c, jobs, nj, s, nsteps);
     }
     return fail("no specialised kernels for this grid");
 }
@@ -789,23 +799,33 @@ static int step_disc_t(lfts_ctx c, const lfts_step_job *jobs, int nj, int s, int
     CKLAUNCH();
     return 0;
 }
-extern "C" int lfts_step_discrete(lfts_ctx c, const lfts_step_job *jobs, int nj, int s, int half, int with_fac) {
-    if (!c || !jobs) return fail("null argument");
-    if (nj <= 0) return 0;
-    if (nj > 65535) return fail("too many jobs in one launch (max 65535)");
+static int steps_discrete(lfts_ctx c, const lfts_step_job *jobs, int nj, int s0, int nsteps, int half, int with_fac) {
     half = half ? 1 : 0;
-    c->launches += 3;
+    if ((!with_fac || (!c->fastN && !c->any)) && nsteps > 1) {  // no seam without the factor, nor in the kernels for large planes
+        for (int s = s0; s < s0 + nsteps; s++) {
+            const int rc = steps_discrete(c, jobs, nj, s, 1, half, with_fac);
+            if (rc) return rc;
+        }
+        return 0;
+    }
+    c->launches += 1 + 2 * (long long)nsteps;
     if (c->fastN)
-        return c->prec == 8 ? step_fast_dispatch<double>(c, jobs, nj, s, 1, 1, half, with_fac)
-                            : step_fast_dispatch<float>(c, jobs, nj, s, 1, 1, half, with_fac);
+        return c->prec == 8 ? step_fast_dispatch<double>(c, jobs, nj, s0, nsteps, 1, half, with_fac)
+                            : step_fast_dispatch<float>(c, jobs, nj, s0, nsteps, 1, half, with_fac);
     if (c->any) {
-        any_step_discrete(c->any, c->stream, jobs, nj, s, half, with_fac);
+        any_steps_discrete(c->any, c->stream, jobs, nj, s0, nsteps, half, with_fac);
         CKLAUNCH();
         return 0;
     }
     if (c->prec == 8)
-        return c->gen ? step_disc_t<double, true>(c, jobs, nj, s, half, with_fac) : step_disc_t<double, false>(c, jobs, nj, s, half, with_fac);
-    return c->gen ? step_disc_t<float, true>(c, jobs, nj, s, half, with_fac) : step_disc_t<float, false>(c, jobs, nj, s, half, with_fac);
+        return c->gen ? step_disc_t<double, true>(c, jobs, nj, s0, half, with_fac) : step_disc_t<double, false>(c, jobs, nj, s0, half, with_fac);
+    return c->gen ? step_disc_t<float, true>(c, jobs, nj, s0, half, with_fac) : step_disc_t<float, false>(c, jobs, nj, s0, half, with_fac);
+}
+extern "C" int lfts_step_discrete(lfts_ctx c, const lfts_step_job *jobs, int nj, int s, int half, int with_fac) {
+    if (!c || !jobs) return fail("null argument");
+    if (nj <= 0) return 0;
+    if (nj > 65535) return fail("too many jobs in one launch (max 65535)");
+    return steps_discrete(c, jobs, nj, s, 1, half, with_fac);
 }
 
 // ---------------------------------------------------------------- sweeps
@@ -837,11 +857,7 @@ extern "C" int lfts_sweep_discrete(lfts_ctx c, const lfts_step_job *jobs, int nj
         c->launches += 1;
         return 0;
     }
-    for (int s = s0; s < s0 + nsteps; s++) {
-        const int rc = lfts_step_discrete(c, jobs, nj, s, half, with_fac);
-        if (rc) return rc;
-    }
-    return 0;
+    return steps_discrete(c, jobs, nj, s0, nsteps, half, with_fac);
 }
 
 // ---------------------------------------------------------------- junctions

@@ -99,7 +99,7 @@ template <typename K> bool allow(K kernel, int max_smem, bool cluster = false) {
 }
 template <typename T> bool allow_all(int max_smem) {
     return allow(any::ka_plane_forward<T, true>, max_smem) && allow(any::ka_plane_forward<T, false>, max_smem) &&
-           allow(any::ka_plane_mid<T>, max_smem) && allow(any::ka_plane_inverse<T, true>, max_smem) &&
+           allow(any::ka_plane_mid<T, false>, max_smem) && allow(any::ka_plane_mid<T, true>, max_smem) && allow(any::ka_plane_inverse<T, true>, max_smem) &&
            allow(any::ka_plane_inverse<T, false>, max_smem) && allow(any::ka_plane_seam<T>, max_smem) && allow(any::ka_xpass<T, 1>, max_smem) &&
            allow(any::ka_xpass<T, 2>, max_smem) && allow(any::ka_xpass_forward<T>, max_smem) && allow(any::ka_xstress<T>, max_smem) &&
            allow(any::ka_sweep_continuous<T>, max_smem, true) && allow(any::ka_sweep_discrete<T>, max_smem, true);
@@ -268,8 +268,8 @@ template <typename T> void steps_continuous(const AnyGrid *a, cudaStream_t st, c
     plane_forward<T, true>(a, st, jobs, nj, s0, FM_FAC_SQ, FM_FAC, 0);
     for (int s = s0; s < s0 + nsteps; s++) {
         xpass<T, 2>(a, st, jobs, nj, 0, 0, 1);
-        launch_after(any::ka_plane_mid<T>, dim3(mid_ctas, nj), plane_threads(a, mid_ctas * nj, km * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, km),
-                     st, g, jobs, 1, stack(g, km));
+        launch_after(any::ka_plane_mid<T, false>, dim3(mid_ctas, nj), plane_threads(a, mid_ctas * nj, km * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, km),
+                     st, g, jobs, 1, 0, stack(g, km));
         xpass<T, 1>(a, st, jobs, nj, 1, 1, 1);
         if (s + 1 < s0 + nsteps)
             launch_after(any::ka_plane_seam<T>, dim3(ctas, nj), plane_threads(a, ctas * nj, k * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, k), st,
@@ -278,10 +278,19 @@ template <typename T> void steps_continuous(const AnyGrid *a, cudaStream_t st, c
             plane_inverse<T, true>(a, st, jobs, nj, s, 0, 0);
     }
 }
-template <typename T> void step_discrete(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s, int half, int wf) {
-    plane_forward<T, false>(a, st, jobs, nj, s, FM_NONE, 0, 0);
-    xpass<T, 1>(a, st, jobs, nj, 0, half, half);
-    plane_inverse<T, false>(a, st, jobs, nj, s, 0, wf ? FM_FAC : FM_NONE);
+template <typename T> void steps_discrete(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps, int half, int wf) {
+    using C = typename CT<T>::type;
+    const Plan &g = a->p;
+    const int pairs = ceil_div(g.n0, 2), km = stack_planes<C>(a, pairs, nj), ctas = ceil_div(pairs, km);
+    plane_forward<T, false>(a, st, jobs, nj, s0, FM_NONE, 0, 0);
+    for (int s = s0; s < s0 + nsteps; s++) {
+        xpass<T, 1>(a, st, jobs, nj, 0, half, half);
+        if (s + 1 < s0 + nsteps)
+            launch_after(any::ka_plane_mid<T, true>, dim3(ctas, nj), plane_threads(a, ctas * nj, km * g.n1 * g.n2), any::PlaneBuf<C>::bytes(g, km), st,
+                         g, jobs, 0, s, stack(g, km));
+        else
+            plane_inverse<T, false>(a, st, jobs, nj, s, 0, wf ? FM_FAC : FM_NONE);
+    }
 }
 template <typename T> void xforward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj) {
     using C = typename CT<T>::type;
@@ -346,8 +355,8 @@ void any_destroy(AnyGrid *a) {
 void any_steps_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps) {
     a->prec == 8 ? steps_continuous<double>(a, st, jobs, nj, s0, nsteps) : steps_continuous<float>(a, st, jobs, nj, s0, nsteps);
 }
-void any_step_discrete(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s, int half, int wf) {
-    a->prec == 8 ? step_discrete<double>(a, st, jobs, nj, s, half, wf) : step_discrete<float>(a, st, jobs, nj, s, half, wf);
+void any_steps_discrete(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps, int half, int wf) {
+    a->prec == 8 ? steps_discrete<double>(a, st, jobs, nj, s0, nsteps, half, wf) : steps_discrete<float>(a, st, jobs, nj, s0, nsteps, half, wf);
 }
 void any_planes_forward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj) {
     a->prec == 8 ? plane_forward<double, false>(a, st, jobs, nj, 0, FM_NONE, 0, 0, false) : plane_forward<float, false>(a, st, jobs, nj, 0, FM_NONE, 0, 0, false);

@@ -210,8 +210,11 @@ __device__ __forceinline__ void load_packed(const Plan &g, const C *__restrict__
 
 // ------------------------------------------------------------------------
 // K3: inverse zy of planes 2p, 2p + 1, multiply by fac^2, forward zy, in place
-template <typename T>
-__global__ void __launch_bounds__(NT_MAX) ka_plane_mid(const __grid_constant__ Plan g, const lfts_step_job *__restrict__ jobs, int spec_idx, Stack sk) {
+// (SEAM: the discrete step's seam, K5 of step s and K1 of step s + 1: the factor is fac
+// and the product, q', also goes to memory)
+template <typename T, bool SEAM>
+__global__ void __launch_bounds__(NT_MAX) ka_plane_mid(const __grid_constant__ Plan g, const lfts_step_job *__restrict__ jobs, int spec_idx, int s,
+                                                       Stack sk) {
     using C = typename CT<T>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PlaneBuf<C> sm(smem_raw, g, sk.planes);
@@ -225,13 +228,18 @@ __global__ void __launch_bounds__(NT_MAX) ka_plane_mid(const __grid_constant__ P
     __syncthreads();
     plane_inverse(g, sm.buf, sk, sm.twy, sm.twz);
     const T *fac = (const T *)jb.fac + (long long)x0 * area;
+    T *qout = SEAM ? (T *)jb.out + s * jb.out_stride + (long long)x0 * area : nullptr;
     for (int i = threadIdx.x; i < np * area; i += blockDim.x) {
         const Point pt = point_at(g, i, sm.iy, sm.iz);
         const int src = (2 * pt.p * g.n1 + pt.y) * g.n2 + pt.t;
         const T ea = fac[src], eb = 2 * pt.p + 1 < nx ? fac[src + area] : (T)0;
         C z = sm.buf[pt.o];
-        z.x *= ea * ea;
-        z.y *= eb * eb;
+        z.x *= SEAM ? ea : ea * ea;
+        z.y *= SEAM ? eb : eb * eb;
+        if (SEAM) {
+            qout[src] = z.x;
+            if (2 * pt.p + 1 < nx) qout[src + area] = z.y;
+        }
         sm.buf[pt.o] = z;
     }
     __syncthreads();

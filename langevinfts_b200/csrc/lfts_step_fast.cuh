@@ -323,8 +323,10 @@ __device__ __forceinline__ void fload_inverse_y(const GridPlan &g, const lfts_st
 
 // ------------------------------------------------------------------------
 // K3 (fast): inverse zy, multiply by e = fac^2, forward zy, in place on a spectrum slot
-template <typename T, int N, int NT = NTHR>
-__global__ void __launch_bounds__(NT) kf_plane_mid(GridPlan g, const lfts_step_job *__restrict__ jobs, int spec_idx) {
+// (SEAM: the discrete step's seam, K5 of step s and K1 of step s + 1: the factor is fac
+// and the product, q', also goes to memory)
+template <typename T, int N, int NT = NTHR, bool SEAM = false>
+__global__ void __launch_bounds__(NT) kf_plane_mid(GridPlan g, const lfts_step_job *__restrict__ jobs, int spec_idx, int s) {
     using C = typename CT<T>::type;
     using SM = FSmem<C, N, 1, 1, NT>;
     constexpr int NZC = SM::NZC, PL = SM::PL, ZB = SM::ZB, NU = N / 2;
@@ -342,6 +344,7 @@ __global__ void __launch_bounds__(NT) kf_plane_mid(GridPlan g, const lfts_step_j
     __syncthreads();
     fload_inverse_y<C, N, 1, NT>(g, jb, spec_idx, P, stw);
     const T *fac = (const T *)jb.fac + (long long)x * N * N;
+    T *qout = SEAM ? (T *)jb.out + s * jb.out_stride + (long long)x * N * N : nullptr;
     C *zw = zl + warp * ZB * PL;
     constexpr int PER = (N + 31) / 32;
     for (int u0 = warp * ZB; u0 < NU; u0 += (NT / 32) * ZB) {
@@ -376,8 +379,13 @@ __global__ void __launch_bounds__(NT) kf_plane_mid(GridPlan g, const lfts_step_j
                 const int t = lane + 32 * i;
                 if (t < N) {
                     const C z = zw[b * PL + LZ::off(t)];
-                    v[i].x = z.x * ea[b][i] * ea[b][i];
-                    v[i].y = z.y * eb[b][i] * eb[b][i];
+                    v[i].x = SEAM ? z.x * ea[b][i] : z.x * ea[b][i] * ea[b][i];
+                    v[i].y = SEAM ? z.y * eb[b][i] : z.y * eb[b][i] * eb[b][i];
+                    if (SEAM) {
+                        T *row = qout + 2 * (u0 + b) * N + t;
+                        row[0] = v[i].x;
+                        row[N] = v[i].y;
+                    }
                 }
             }
             __syncwarp();

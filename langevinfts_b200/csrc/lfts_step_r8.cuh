@@ -545,8 +545,10 @@ __global__ void __launch_bounds__(NTHR, 3) kp_xpass(GridPlan g, const lfts_step_
 
 // ------------------------------------------------------------------------
 // K3: inverse zy, multiply by e = fac^2, forward zy, in place on slot spec_idx
-template <typename T>
-__global__ void __launch_bounds__(NTHR, (sizeof(T) == 4 ? LFTS_R8_MINB_F32 : LFTS_R8_MINB)) kr_plane_mid(GridPlan g, const lfts_step_job *__restrict__ jobs, int spec_idx) {
+// (SEAM: the discrete step's seam, K5 of step s and K1 of step s + 1: the factor is fac
+// and the product, q', also goes to memory)
+template <typename T, bool SEAM = false>
+__global__ void __launch_bounds__(NTHR, (sizeof(T) == 4 ? LFTS_R8_MINB_F32 : LFTS_R8_MINB)) kr_plane_mid(GridPlan g, const lfts_step_job *__restrict__ jobs, int spec_idx, int s) {
     using C = typename CT<T>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *P = (C *)smem_raw;
@@ -563,6 +565,7 @@ __global__ void __launch_bounds__(NTHR, (sizeof(T) == 4 ? LFTS_R8_MINB_F32 : LFT
     {
         const int u = grp;
         const T *frow = fac + u * N + j;
+        T *qrow = SEAM ? (T *)jb.out + s * jb.out_stride + (long long)x * N * N + u * N + j : nullptr;
         T ea[8], eb[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) {
@@ -576,8 +579,12 @@ __global__ void __launch_bounds__(NTHR, (sizeof(T) == 4 ? LFTS_R8_MINB_F32 : LFT
         fft64<+1>(a, RowX<C>{P, u}, j, wi, mask);
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-            a[k].x = a[k].x * ea[k] * ea[k];
-            a[k].y = a[k].y * eb[k] * eb[k];
+            a[k].x = SEAM ? a[k].x * ea[k] : a[k].x * ea[k] * ea[k];
+            a[k].y = SEAM ? a[k].y * eb[k] : a[k].y * eb[k] * eb[k];
+            if (SEAM) {
+                qrow[8 * k] = a[k].x;
+                qrow[32 * N + 8 * k] = a[k].y;
+            }
         }
         fft64<-1>(a, RowX<C>{P, u}, j, wf, mask);
 #pragma unroll
