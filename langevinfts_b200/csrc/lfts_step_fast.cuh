@@ -56,7 +56,14 @@ __host__ __device__ constexpr int stw_offset(int n, int s) {
 }
 __host__ __device__ constexpr int stw_size(int n) { return stw_offset(n, nrad(n)); }
 __host__ __device__ constexpr int padded(int n) { return n + n / 8 + 1; }
-__host__ __device__ constexpr int zlines(int n) { return (256 / n) < 1 ? 1 : (256 / n); }
+// z-lines a warp transforms at a time: at most what keeps 32 lanes in a radix-8 stage
+// (256 points; 48-point lines six), but no more than the block's units over its warps,
+// so that a small plane leaves no warp without lines (32^3: with 8 lines a warp 4 of 8
+// warps had rows in K1 and K5, and 2 of 8 in the mid kernel)
+__host__ __device__ constexpr int zlines(int n, int units, int warps) {
+    const int most = n == 48 ? 6 : 256 / n < 1 ? 1 : 256 / n, share = (units + warps - 1) / warps;
+    return most < share ? most : share;
+}
 
 template <int N>
 __device__ __forceinline__ int perm_ct(int t) {
@@ -146,7 +153,7 @@ template <typename C, int N, int NBR, int NZL, int NT = NTHR>
 struct FSmem {
     static constexpr int NZC = N / 2 + 1;
     static constexpr int PL = padded(N);
-    static constexpr int ZB = zlines(N);
+    static constexpr int ZB = zlines(N, NBR == 2 ? N : N / 2, NT / 32);
     static constexpr size_t P_ELEMS = (size_t)NBR * N * NZC;
     static constexpr size_t Z_ELEMS = (size_t)NZL * (NT / 32) * ZB * PL;
     static constexpr size_t BYTES = sizeof(C) * (P_ELEMS + Z_ELEMS + stw_size(N) + 1);

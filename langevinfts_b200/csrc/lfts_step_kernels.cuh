@@ -1,4 +1,6 @@
-// Fused pseudo-spectral step kernels (sm_100a).
+// Fused pseudo-spectral step kernels (sm_100a): what every family shares, and the
+// runtime-radix kernels k_*, which serve the planes that the any-extent kernels
+// (lfts_step_any.cuh) cannot hold in shared memory.
 //
 // One continuous Richardson step (reference: CudaSolverPseudo.cu:345-412, six
 // cuFFT calls and ~12 pointwise kernels) is five launches here, each a single
