@@ -148,7 +148,7 @@ def reference_sample(n_iter, threads, timeout=900, workload="diblock64"):
     r = subprocess.run([sys.executable, os.path.abspath(__file__), "--ref-sample", str(n_iter), "--threads", str(threads),
                         "--workload", workload],
                        env=env, preexec_fn=unlimited_stack, capture_output=True, text=True, timeout=timeout)
-    if r.returncode != 0:
+    if r.returncode != 0 or not r.stdout.strip():  # no output: the reference build is missing
         sys.stderr.write(r.stdout[-2000:] + r.stderr[-2000:])
         return None
     return tuple(json.loads(r.stdout.strip().splitlines()[-1]))
