@@ -187,6 +187,11 @@ int lfts_step_impl(lfts_ctx ctx, char *name, size_t cap);
  * Named kernels other than "cluster-<n>" also run the sweeps step by step.
  * Not during a graph capture.  No counterpart in the reference. */
 int lfts_set_step_impl(lfts_ctx ctx, const char *name);
+/* Radices of the any-extent kernels' n-point transform, outermost first: 2 to 13
+ * and 16 in registers, primes above 13 (up to 61) as pair sums.  radices has room
+ * for cap, *count receives their number.  Host only.  No counterpart in the
+ * reference (cuFFT plans there). */
+int lfts_transform_radices(int n, int *radices, int cap, int *count);
 /* Discrete chain: out = [fac *] F^-1[ b * F[in] ] with b = bond (half=0) or
  * bond_half (half=1), multiplied by fac when with_fac=1.  (half=0, with_fac=1)
  * replaces advance_propagator_discrete (CudaSolverPseudo.cu:413-450);

@@ -102,6 +102,7 @@ _SIGS = {
     "lfts_autotune": [C.c_void_p, C.c_int, C.c_int, C.c_char_p, C.c_size_t],
     "lfts_step_impl": [C.c_void_p, C.c_char_p, C.c_size_t],
     "lfts_realspace_tables": [C.c_void_p, C.c_double, C.c_double, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p],
+    "lfts_transform_radices": [C.c_int, C.POINTER(C.c_int), C.c_int, C.POINTER(C.c_int)],
     "lfts_step_realspace": [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int],
     "lfts_set_step_impl": [C.c_void_p, C.c_char_p],
     "lfts_graph_while_begin": [C.c_void_p, C.POINTER(C.c_ulonglong)],

@@ -1,6 +1,7 @@
 // Host side of the any-extent step kernels (lfts_step_any.cu).
 #pragma once
 #include <string>
+#include <vector>
 
 #include <cuda_runtime.h>
 
@@ -14,6 +15,9 @@ struct AnyGrid;  // plan, device tables and launch limits of one grid and precis
 // or on a CUDA error (err says which).  axis extents as the context pads them.
 AnyGrid *any_create(int prec, const int n[3], int nsm, int max_smem, std::string &err);
 void any_destroy(AnyGrid *a);
+// Radices of an n-point transform, outermost first: register radices (2 .. 13, 16) and
+// primes above 13; false when a prime is too large for the kernels.
+bool any_radices(int n, std::vector<int> &r);
 
 void any_steps_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps);
 void any_steps_discrete(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps, int half, int with_fac);

@@ -1591,6 +1591,17 @@ extern "C" int lfts_set_step_impl(lfts_ctx c, const char *name) {
     return fail("step implementation \"" + n + "\" is not available for this context");
 }
 
+extern "C" int lfts_transform_radices(int n, int *radices, int cap, int *count) {
+    if (!radices || !count) return fail("null argument");
+    if (n < 1 || n > LFTS_MAX_AXIS) return fail("grid extent " + std::to_string(n) + " is outside [1, 1024]");
+    std::vector<int> r;
+    if (!any_radices(n, r)) return fail("grid extent " + std::to_string(n) + " has a prime factor > 64");
+    if ((int)r.size() > cap) return fail("the plan has " + std::to_string(r.size()) + " radices");
+    std::copy(r.begin(), r.end(), radices);
+    *count = (int)r.size();
+    return 0;
+}
+
 extern "C" int lfts_step_impl(lfts_ctx c, char *name, size_t cap) {
     if (!c || !name || cap == 0) return fail("null argument");
     std::string n = c->r8 ? (c->xcap ? "register-64 xcap" + std::to_string(c->xcap) : std::string("register-64"))

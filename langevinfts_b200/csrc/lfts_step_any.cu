@@ -23,7 +23,10 @@ struct AnyGrid {
 namespace {
 using any::Plan;
 
-// Fewest stages first, then the smallest sum of radices; outermost radix the largest.
+// Fewest stages first, then the smallest sum of radices, radices never rising from the
+// outermost on: every product of the primes up to 13 has such an order, so a branch that
+// its cap leaves without a radix is a dead end (an odd composite taken there as a prime
+// made 98 a radix-49 pair sum instead of 7 x 7 x 2).
 void best_radices(int n, std::vector<int> &cur, std::vector<int> &best, int most) {
     if (n == 1) {
         auto sum = [](const std::vector<int> &v) { int s = 0; for (int x : v) s += x; return s; };
@@ -32,42 +35,17 @@ void best_radices(int n, std::vector<int> &cur, std::vector<int> &best, int most
     }
     if (!best.empty() && cur.size() >= best.size()) return;
     static const int regs[] = {16, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
-    bool any_reg = false;
     for (int r : regs)
         if (r <= most && n % r == 0) {
-            any_reg = true;
             cur.push_back(r);
             best_radices(n / r, cur, best, r);
             cur.pop_back();
         }
-    if (any_reg) return;
-    for (int q = 17; q <= n; q += 2)
-        if (n % q == 0) {
-            cur.push_back(q);
-            best_radices(n / q, cur, best, most);
-            cur.pop_back();
-            return;
-        }
 }
 
 bool make_axis(int n, any::Axis &ax, std::vector<short> &perm, std::vector<short> &iperm) {
-    // primes above 13 go innermost (span 1: no twiddles)
-    std::vector<int> big, cur, r;
-    int m = n;
-    for (int q = 17; q <= m; q += 2)
-        while (m % q == 0) {
-            bool prime = true;
-            for (int d = 3; d * d <= q; d += 2) prime = prime && q % d;
-            if (!prime) break;
-            big.push_back(q);
-            m /= q;
-        }
-    if (m > 1) best_radices(m, cur, r, any::MAX_REG_RADIX);
-    for (int q : big) {
-        if (q > LFTS_MAX_RADIX) return false;
-        r.push_back(q);
-    }
-    if ((int)r.size() > any::MAXF) return false;
+    std::vector<int> r;
+    if (!any_radices(n, r)) return false;
     ax.n = n;
     ax.nf = (int)r.size();
     int span = n;
@@ -322,6 +300,27 @@ template <typename T> int sweep_discrete(const AnyGrid *a, cudaStream_t st, cons
     return (int)cudaLaunchKernelEx(&cfg, any::ka_sweep_discrete<T>, a->p, s.w, jobs, s0, n, half, wf);
 }
 }  // namespace
+
+bool any_radices(int n, std::vector<int> &r) {
+    // primes above 13 go innermost (span 1: no twiddles)
+    std::vector<int> big, cur;
+    int m = n;
+    for (int q = 17; q <= m; q += 2)
+        while (m % q == 0) {
+            bool prime = true;
+            for (int d = 3; d * d <= q; d += 2) prime = prime && q % d;
+            if (!prime) break;
+            big.push_back(q);
+            m /= q;
+        }
+    r.clear();
+    if (m > 1) best_radices(m, cur, r, any::MAX_REG_RADIX);
+    for (int q : big) {
+        if (q > LFTS_MAX_RADIX) return false;
+        r.push_back(q);
+    }
+    return (int)r.size() <= any::MAXF;
+}
 
 AnyGrid *any_create(int prec, const int n[3], int nsm, int max_smem, std::string &err) {
     auto *a = new AnyGrid();
