@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(NT) kf_plane_forward(GridPlan g, const lfts_st
     C *stw = zl + SM::Z_ELEMS;
     load_stw<C, N, NT>(stw, g.stw);
     grid_wait();
-    const lfts_step_job jb = jobs[blockIdx.y];
+    const lfts_step_job jb = job_at(jobs, blockIdx.y);
     if (jb.active && !jb.active[jb.replica]) return;
     const int x = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long poff = (long long)x * N * N;
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(NTHR) kf_xpass(GridPlan g, const lfts_step_job
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *tile = (C *)smem_raw;
     C *stw = tile + NBR * N * TJ;
-    const lfts_step_job jb = jobs[blockIdx.y];
+    const lfts_step_job jb = job_at(jobs, blockIdx.y);
     load_stw<C, N>(stw, g.stw);
     grid_wait();
     if (jb.active && !jb.active[jb.replica]) return;
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(NT) kf_plane_mid(GridPlan g, const lfts_step_j
     C *P = (C *)smem_raw;
     C *zl = P + SM::P_ELEMS;
     C *stw = zl + SM::Z_ELEMS;
-    const lfts_step_job jb = jobs[blockIdx.y];
+    const lfts_step_job jb = job_at(jobs, blockIdx.y);
     load_stw<C, N, NT>(stw, g.stw);
     grid_wait();
     if (jb.active && !jb.active[jb.replica]) return;
@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(NT) kf_plane_inverse(GridPlan g, const lfts_st
     C *P = (C *)smem_raw;
     C *zl = P + SM::P_ELEMS;
     C *stw = zl + SM::Z_ELEMS;
-    const lfts_step_job jb = jobs[blockIdx.y];
+    const lfts_step_job jb = job_at(jobs, blockIdx.y);
     load_stw<C, N, NT>(stw, g.stw);
     grid_wait();
     if (jb.active && !jb.active[jb.replica]) return;
@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(NT) kf_plane_seam(GridPlan g, const lfts_step_
     C *P = (C *)smem_raw;
     C *zl = P + SM::P_ELEMS;
     C *stw = zl + SM::Z_ELEMS;
-    const lfts_step_job jb = jobs[blockIdx.y];
+    const lfts_step_job jb = job_at(jobs, blockIdx.y);
     load_stw<C, N, NT>(stw, g.stw);
     grid_wait();
     if (jb.active && !jb.active[jb.replica]) return;

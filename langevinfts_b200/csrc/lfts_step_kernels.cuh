@@ -31,6 +31,23 @@ constexpr int NWARP = NTHR / 32;
 // (64^3 FP64 33.1 -> 32.1 us, 31 x 49 x 23 49.1 -> 46.7, 32^3 FP32 x 32 jobs 45.9 -> 44.1).
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// A job of the array, its pointers known to lie in global memory.  Read plainly, the
+// pointers are generic to the compiler once grid_wait() stands between the job and their
+// use; loads through them might then alias the stores to shared memory between them and
+// are issued one at a time.  Microseconds a launch, FP64, with plain and with stated
+// pointers: kf_plane_inverse<1> 96^3, 16 jobs 165 and 137; kf_plane_inverse<2> 48^3, 128
+// jobs 323 and 272; kf_xpass<2> 32^3, 128 jobs 61 and 52.
+__device__ __forceinline__ lfts_step_job job_at(const lfts_step_job *__restrict__ jobs, int i) {
+    const lfts_step_job jb = jobs[i];
+    __builtin_assume(__isGlobal(jb.in));
+    __builtin_assume(__isGlobal(jb.out));
+    __builtin_assume(__isGlobal(jb.fac));
+    __builtin_assume(__isGlobal(jb.bond));
+    __builtin_assume(__isGlobal(jb.bond_half));
+    __builtin_assume(__isGlobal(jb.spec));
+    return jb;
+}
+
 // Launch with the programmatic edge to the kernel before it in the stream.
 template <typename... P, typename... A>
 inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
