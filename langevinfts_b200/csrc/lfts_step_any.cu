@@ -13,6 +13,7 @@ namespace lfts {
 struct AnyGrid {
     any::Plan p;
     int prec = 8, nsm = 148, max_smem = 0;
+    int stress_smem = 0;  // dynamic shared memory left to ka_xstress by its static reduction scratch
     void *tables = nullptr;
     // resident clusters of 1, 2, 4, 8, 16 CTAs, estimated (0: no fit); the device's own
     // answer is asked for once, for a size about to be used: it takes a third of a millisecond
@@ -68,11 +69,14 @@ bool make_axis(int n, any::Axis &ax, std::vector<short> &perm, std::vector<short
     return true;
 }
 
-template <typename K> bool allow(K kernel, int max_smem, bool cluster = false) {
+// dynamic shared memory a kernel may have: the block's less its own static part
+template <typename K> int dynamic_limit(K kernel, int max_smem) {
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, kernel) != cudaSuccess) return false;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)fa.sharedSizeBytes) != cudaSuccess)
-        return false;
+    return cudaFuncGetAttributes(&fa, kernel) == cudaSuccess ? max_smem - (int)fa.sharedSizeBytes : 0;
+}
+template <typename K> bool allow(K kernel, int max_smem, bool cluster = false) {
+    const int limit = dynamic_limit(kernel, max_smem);
+    if (limit <= 0 || cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) return false;
     return !cluster || cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
 }
 template <typename T> bool allow_all(int max_smem) {
@@ -183,6 +187,7 @@ template <typename T> bool setup(AnyGrid *a, std::string &err) {
         err = std::string("transform setup: ") + cudaGetErrorString(cudaGetLastError());
         return false;
     }
+    a->stress_smem = dynamic_limit(any::ka_xstress<T>, a->max_smem);
     for (int k = 0; k < 5; k++) {
         a->clusters_cont[k] = estimate_clusters(a, true, 1 << k);
         a->clusters_disc[k] = estimate_clusters(a, false, 1 << k);
@@ -204,12 +209,13 @@ int plane_threads(const AnyGrid *a, int ctas, int points) {
     const int most = ctas <= a->nsm ? any::NT_MAX : 256;
     return std::min(most, std::max(64, (points / 4 + 31) / 32 * 32));
 }
-template <typename C> int tile_columns(const AnyGrid *a, int nbr, int nj) {
+// limit: dynamic shared memory of the kernel that takes the tile
+template <typename C> int tile_columns(const AnyGrid *a, int nbr, int nj, int limit) {
     const Plan &g = a->p;
     int tj = sizeof(C) == 16 ? 16 : 32;
     const int cols = g.n1 * g.nzc;
     // narrower tiles (still whole 64-byte rows) when wide ones leave SMs without work or do not fit
-    while (tj > 4 && (any::TileBuf<C>::bytes(g, nbr * tj) > (size_t)a->max_smem ||
+    while (tj > 4 && (any::TileBuf<C>::bytes(g, nbr * tj) > (size_t)limit ||
                       ((long long)ceil_div(cols, tj) * nj < a->nsm && tj * sizeof(C) > 128)))
         tj /= 2;
     return tj;
@@ -235,7 +241,7 @@ template <typename T, bool TWO> void plane_inverse(const AnyGrid *a, cudaStream_
 template <typename T, int NBR> void xpass(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int spec, int b0, int b1) {
     using C = typename CT<T>::type;
     const Plan &g = a->p;
-    const int tj = tile_columns<C>(a, NBR, nj), ctas = ceil_div(g.n1 * g.nzc, tj);
+    const int tj = tile_columns<C>(a, NBR, nj, a->max_smem), ctas = ceil_div(g.n1 * g.nzc, tj);
     launch_after(any::ka_xpass<T, NBR>, dim3(ctas, nj), plane_threads(a, ctas * nj, g.n0 * tj * NBR), any::TileBuf<C>::bytes(g, NBR * tj), st, g, jobs, spec, b0, b1, tj, any::div_mul(tj), any::div_mul(NBR * tj));
 }
 template <typename T> void steps_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps) {
@@ -273,7 +279,7 @@ template <typename T> void steps_discrete(const AnyGrid *a, cudaStream_t st, con
 template <typename T> void xforward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj) {
     using C = typename CT<T>::type;
     const Plan &g = a->p;
-    const int tj = tile_columns<C>(a, 1, nj), ctas = ceil_div(g.n1 * g.nzc, tj);
+    const int tj = tile_columns<C>(a, 1, nj, a->max_smem), ctas = ceil_div(g.n1 * g.nzc, tj);
     any::ka_xpass_forward<T><<<dim3(ctas, nj), plane_threads(a, ctas * nj, g.n0 * tj), any::TileBuf<C>::bytes(g, tj), st>>>(
         g, jobs, tj, any::div_mul(tj), any::div_mul(tj));
 }
@@ -281,7 +287,7 @@ template <typename T> void xstress(const AnyGrid *a, cudaStream_t st, const lfts
                                    const double *basis, double *partials) {
     using C = typename CT<T>::type;
     const Plan &g = a->p;
-    const int tj = tile_columns<C>(a, 2, nj);
+    const int tj = tile_columns<C>(a, 2, nj, a->stress_smem);
     any::ka_xstress<T><<<dim3(ceil_div(g.n1 * g.nzc, tj), nj), NTHR, any::TileBuf<C>::bytes(g, 2 * tj), st>>>(
         g, sj, jobs, basis, tj, any::div_mul(tj), any::div_mul(2 * tj), partials);
 }
@@ -364,7 +370,7 @@ void any_xpass_forward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *j
     a->prec == 8 ? xforward<double>(a, st, jobs, nj) : xforward<float>(a, st, jobs, nj);
 }
 int any_stress_tiles(const AnyGrid *a, int nj) {
-    return ceil_div(a->p.n1 * a->p.nzc, a->prec == 8 ? tile_columns<double2>(a, 2, nj) : tile_columns<float2>(a, 2, nj));
+    return ceil_div(a->p.n1 * a->p.nzc, a->prec == 8 ? tile_columns<double2>(a, 2, nj, a->stress_smem) : tile_columns<float2>(a, 2, nj, a->stress_smem));
 }
 void any_xstress(const AnyGrid *a, cudaStream_t st, const lfts_step_job *sj, const lfts_stress_job *jobs, int nj, const double *basis,
                  double *partials) {
