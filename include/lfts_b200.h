@@ -206,6 +206,10 @@ int lfts_step_discrete(lfts_ctx ctx, const lfts_step_job *jobs, int njobs, int s
  * after the other.  No counterpart in the reference. */
 int lfts_sweep_continuous(lfts_ctx ctx, const lfts_step_job *jobs, int njobs, int s0, int nsteps);
 int lfts_sweep_discrete(lfts_ctx ctx, const lfts_step_job *jobs, int njobs, int s0, int nsteps, int half, int with_fac);
+/* CTAs per job of the cluster launch that a sweep of njobs jobs is on this context
+ * (0: steps of separate launches).  It depends on the grid, the precision, njobs and
+ * lfts_set_step_impl only, never on earlier calls.  No counterpart in the reference. */
+int lfts_sweep_size(lfts_ctx ctx, int continuous, int njobs, int *ctas);
 
 /* ---- junctions and initial slices --------------------------------------- */
 

@@ -62,6 +62,7 @@ _SIGS = {
     "lfts_step_discrete": [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int],
     "lfts_sweep_continuous": [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int],
     "lfts_sweep_discrete": [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int],
+    "lfts_sweep_size": [C.c_void_p, C.c_int, C.c_int, C.POINTER(C.c_int)],
     "lfts_junctions": [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p],
     "lfts_dots": [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p],
     "lfts_dots_static": [C.c_int, C.c_longlong, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p],

@@ -33,7 +33,7 @@ void any_xstress(const AnyGrid *a, cudaStream_t st, const lfts_step_job *sj, con
 
 // CTAs per job of the cluster sweep for nj jobs; 0: the grid does not fit or the
 // separate passes are faster.  force: 0 by that rule, else this cluster size where it fits.
-int any_sweep_size(AnyGrid *a, bool continuous, int nj, int force);
+int any_sweep_size(const AnyGrid *a, bool continuous, int nj, int force);
 int any_sweep_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps, int cs);
 int any_sweep_discrete(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps, int half,
                        int with_fac, int cs);

@@ -835,6 +835,12 @@ static int sweep_size(lfts_ctx c, bool continuous, int nj) {
     if (!c->any || c->sweep < 0 || (c->sweep == 0 && c->fastN)) return 0;
     return any_sweep_size(c->any, continuous, nj, c->sweep);
 }
+extern "C" int lfts_sweep_size(lfts_ctx c, int continuous, int nj, int *ctas) {
+    if (!c || !ctas) return fail("null argument");
+    if (nj < 1 || nj > 65535) return fail("sweep size: njobs must be 1..65535");
+    *ctas = sweep_size(c, continuous != 0, nj);
+    return 0;
+}
 extern "C" int lfts_sweep_continuous(lfts_ctx c, const lfts_step_job *jobs, int nj, int s0, int nsteps) {
     if (!c || !jobs) return fail("null argument");
     if (nj <= 0 || nsteps <= 0) return 0;

@@ -15,10 +15,9 @@ struct AnyGrid {
     int prec = 8, nsm = 148, max_smem = 0;
     int stress_smem = 0;  // dynamic shared memory left to ka_xstress by its static reduction scratch
     void *tables = nullptr;
-    // resident clusters of 1, 2, 4, 8, 16 CTAs, estimated (0: no fit); the device's own
-    // answer is asked for once, for a size about to be used: it takes a third of a millisecond
+    // clusters of 1, 2, 4, 8, 16 CTAs the device holds at once (0: no fit), asked of it at
+    // creation, so that the rule below gives a grid and a number of jobs one size for good
     int clusters_cont[5] = {0, 0, 0, 0, 0}, clusters_disc[5] = {0, 0, 0, 0, 0};
-    bool asked_cont[5] = {}, asked_disc[5] = {};
 };
 
 namespace {
@@ -135,6 +134,7 @@ template <typename K> void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAtt
 
 template <typename K> int resident_clusters(const AnyGrid *a, K kernel, bool continuous, int cs) {
     const SweepShape s = sweep_shape(a, continuous, cs);
+    if (s.smem > (size_t)a->max_smem) return 0;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at;
     cluster_config(cfg, &at, kernel, cs, 64, sweep_threads(a, s), s.smem, 0);
@@ -144,13 +144,6 @@ template <typename K> int resident_clusters(const AnyGrid *a, K kernel, bool con
         return 0;
     }
     return n;
-}
-// clusters stay within one of eight groups of SMs; a CTA takes its threads' 128 registers
-int estimate_clusters(const AnyGrid *a, bool continuous, int cs) {
-    const SweepShape s = sweep_shape(a, continuous, cs);
-    if (s.smem > (size_t)a->max_smem) return 0;
-    const int per_sm = (int)std::min<size_t>(512 / sweep_threads(a, s), (size_t)a->max_smem / s.smem);
-    return std::max(1, 8 * (a->nsm / 8 * std::max(per_sm, 1) / cs));
 }
 
 template <typename T> bool setup(AnyGrid *a, std::string &err) {
@@ -189,8 +182,8 @@ template <typename T> bool setup(AnyGrid *a, std::string &err) {
     }
     a->stress_smem = dynamic_limit(any::ka_xstress<T>, a->max_smem);
     for (int k = 0; k < 5; k++) {
-        a->clusters_cont[k] = estimate_clusters(a, true, 1 << k);
-        a->clusters_disc[k] = estimate_clusters(a, false, 1 << k);
+        a->clusters_cont[k] = resident_clusters(a, any::ka_sweep_continuous<T>, true, 1 << k);
+        a->clusters_disc[k] = resident_clusters(a, any::ka_sweep_discrete<T>, false, 1 << k);
     }
     return true;
 }
@@ -382,38 +375,27 @@ void any_xstress(const AnyGrid *a, cudaStream_t st, const lfts_step_job *sj, con
 // step in clusters of 16 against 27.7 (17.7 / 27.9); 256 points 16.2 / 25.4; 24^3 25 / 30;
 // 32^3, 32 768 points, 32.5 / 32.0 (26.6 / 30.4): the lines cross near 1500 (2500) points a
 // CTA.  More clusters than the device holds at once run in waves.
-int any_sweep_size(AnyGrid *a, bool continuous, int nj, int force) {
-    int *res = continuous ? a->clusters_cont : a->clusters_disc;
-    bool *asked = continuous ? a->asked_cont : a->asked_disc;
-    auto ask = [&](int k) {
-        if (res[k] && !asked[k]) {
-            asked[k] = true;
-            res[k] = a->prec == 8 ? (continuous ? resident_clusters(a, any::ka_sweep_continuous<double>, true, 1 << k)
-                                                : resident_clusters(a, any::ka_sweep_discrete<double>, false, 1 << k))
-                                  : (continuous ? resident_clusters(a, any::ka_sweep_continuous<float>, true, 1 << k)
-                                                : resident_clusters(a, any::ka_sweep_discrete<float>, false, 1 << k));
-        }
-        return res[k];
-    };
+int any_sweep_size(const AnyGrid *a, bool continuous, int nj, int force) {
+    const int *res = continuous ? a->clusters_cont : a->clusters_disc;
     if (force) {
         for (int k = 0; k < 5; k++)
-            if (1 << k == force && ask(k)) return force;
+            if (1 << k == force && res[k]) return force;
         return 0;
     }
     const bool f64 = a->prec == 8;
     const double M = (double)a->p.M, part = continuous ? 1.0 : 0.55;
     const double fixed = f64 ? 17.5 : 14.5, per_point = f64 ? 7.3e-3 : 4.8e-3;
     double best = part * (26.0 + nj * M * (f64 ? 5e-5 : 4e-5));
-    int size = -1;
+    int size = 0;
     for (int k = 0; k < 5; k++) {
         if (!res[k]) continue;
         const double t = part * ((nj + res[k] - 1) / res[k]) * (fixed + per_point * M / (1 << k));
         if (t < best) {
             best = t;
-            size = k;
+            size = 1 << k;
         }
     }
-    return size >= 0 && ask(size) ? 1 << size : 0;
+    return size;
 }
 int any_sweep_continuous(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s0, int nsteps, int cs) {
     return a->prec == 8 ? sweep_continuous<double>(a, st, jobs, nj, s0, nsteps, cs) : sweep_continuous<float>(a, st, jobs, nj, s0, nsteps, cs);
