@@ -87,8 +87,8 @@ constexpr int NT = 512;
 template <int DIM, int A, bool FIRST, bool LAST, int W>
 __global__ void __launch_bounds__(NT) k_rs_sweep(GridPlan g, const lfts_step_job *__restrict__ jobs, int s, int src_half) {
     extern __shared__ double sm_rs[];
+    grid_wait();  // before the job array too: FIRST is the first kernel of a step
     const lfts_step_job jb = jobs[blockIdx.y];
-    grid_wait();
     if (jb.active && !jb.active[jb.replica]) return;
     constexpr int ld = W + 1;
     const double *q = (const double *)jb.in + s * jb.in_stride, *fac = (const double *)jb.fac, *tab = (const double *)jb.bond;

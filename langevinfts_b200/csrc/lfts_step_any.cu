@@ -214,7 +214,7 @@ template <typename C> int tile_columns(const AnyGrid *a, int nbr, int nj, int li
     return tj;
 }
 
-// in_step: the job array is older than the kernel before this one
+// in_step: with the programmatic edge of the step kernels (the kernel reads the job array after its wait)
 template <typename T, bool TWO> void plane_forward(const AnyGrid *a, cudaStream_t st, const lfts_step_job *jobs, int nj, int s, int f0, int f1, int spec, bool in_step = true) {
     using C = typename CT<T>::type;
     const Plan &g = a->p;
