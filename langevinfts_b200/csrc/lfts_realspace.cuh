@@ -17,11 +17,13 @@
 // job).  All its threads compute right-hand sides into a shared-memory tile,
 // with accesses to global memory in its order whatever the axis (rows of W + 1
 // doubles keep both orders off each other's banks), one warp then solves, a line
-// a lane, and all threads write the tile back.  The substitutions are one chain of
-// fused multiply-adds each (the reciprocal pivots are folded into the right-hand
-// sides and the off-diagonals beforehand), whose operands come from shared memory
-// ahead of the chain.  One thread a line straight from global memory left 24 CTAs
-// waiting on every element: 72 us a sweep at 48 x 48 x 64, 2 jobs.
+// a lane, and all threads write the tile back.  The substitutions are one chain each,
+// whose operands come from shared memory ahead of it: a fused multiply-add and the
+// product with the reciprocal pivot an element (folding that into the right-hand
+// sides and the off-diagonals takes one operation off the chain, 2 % of a film's
+// step, but rounds a matrix entry that every step applies again: 200 points, 100
+// steps 5.2e-15 off instead of 3.6e-15).  One thread a line straight from global
+// memory left 24 CTAs waiting on every element: 72 us a sweep at 48 x 48 x 64, 2 jobs.
 #pragma once
 #include "lfts_step_kernels.cuh"
 
@@ -65,7 +67,7 @@ __device__ __forceinline__ double eq(const double *q, const double *fac, long lo
 }
 
 // shared memory of a block: the tile and six rows of the axis's tables
-constexpr int T_ROWS = 6;  // l, d, h, l / pivot, ratio, periodic vector
+constexpr int T_ROWS = 6;  // l, d, h, 1 / pivot, ratio, periodic vector
 __host__ __device__ constexpr size_t tile_smem(int n, int W) { return sizeof(double) * ((size_t)n * (W + 1) + T_ROWS * (size_t)n); }
 
 // Flat index of element i of line `line` along padded axis A
@@ -100,7 +102,7 @@ __global__ void __launch_bounds__(NT) k_rs_sweep(GridPlan g, const lfts_step_job
         tl[i] = X.l[i];
         td[i] = X.d[i];
         th[i] = X.h[i];
-        tp[i] = X.l[i] * X.rp[i];
+        tp[i] = X.rp[i];
         tc[i] = X.c[i];
         tv[i] = X.v[i];
     }
@@ -141,14 +143,15 @@ __global__ void __launch_bounds__(NT) k_rs_sweep(GridPlan g, const lfts_step_job
                     tl[i] * Em - th[i] * Ep;
             }
         }
-        tile[i * ld + w] = r * X.rp[i];
+        tile[i * ld + w] = r;
     }
     __syncthreads();
     if (threadIdx.x < nl) {
-        double *x = tile + threadIdx.x, v = x[0];
+        double *x = tile + threadIdx.x, v = x[0] * tp[0];
+        x[0] = v;
 #pragma unroll 8
         for (int i = 1; i < n; i++) {
-            v = x[i * ld] - tp[i] * v;
+            v = (x[i * ld] - tl[i] * v) * tp[i];
             x[i * ld] = v;
         }
 #pragma unroll 8
