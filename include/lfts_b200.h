@@ -179,12 +179,17 @@ int lfts_step_realspace(lfts_ctx ctx, const lfts_step_job *jobs, int njobs, int 
 int lfts_autotune(lfts_ctx ctx, int njobs, int reps, char *report, size_t report_cap);
 /* Name of the context's current step implementation ("register-64",
  * "register-64 xcap2", "register-96", "cubic", "generic"): the default chosen
- * at creation, or lfts_autotune's choice.  No counterpart in the reference. */
+ * at creation, lfts_autotune's choice, or what lfts_set_step_impl set
+ * ("cluster-<n>" included).  Sweeps of small grids with "generic" steps may run as
+ * cluster launches unless that name was set: lfts_sweep_size tells.  No counterpart
+ * in the reference. */
 int lfts_step_impl(lfts_ctx ctx, char *name, size_t cap);
 /* Make name the context's step implementation ("register-64", "register-96",
  * "cubic", "generic", or "cluster-<n>": sweeps as one launch of n-CTA clusters,
  * n = 1, 2, 4, 8 or 16); an error when the context has no such implementation.
- * Named kernels other than "cluster-<n>" also run the sweeps step by step.
+ * A named family runs the sweeps too, as a launch for every pass and, between two
+ * steps, its seam kernel where it has one.  "default" is the context as created:
+ * its most specialised family, sweeps of small grids in clusters by rule.
  * Not during a graph capture.  No counterpart in the reference. */
 int lfts_set_step_impl(lfts_ctx ctx, const char *name);
 /* Radices of the any-extent kernels' n-point transform, outermost first: 2 to 13

@@ -1580,14 +1580,18 @@ extern "C" int lfts_set_step_impl(lfts_ctx c, const char *name) {
         c->r8 = r8;
         c->r12 = r12;
         c->xcap = 0;
-        c->sweep = -1;  // the named kernels, step by step
+        c->sweep = -1;  // the named kernels also in sweeps
         return 0;
     };
-    if (n.rfind("cluster-", 0) == 0 && c->any) {
-        const int cs = std::atoi(n.c_str() + 8);
-        if (any_sweep_size(c->any, true, 1, cs) != cs && any_sweep_size(c->any, false, 1, cs) != cs)
-            return fail("step implementation \"" + n + "\" is not available for this context");
-        c->sweep = cs;
+    if (c->any)
+        for (int cs = 1; cs <= 16; cs *= 2)
+            if (n == "cluster-" + std::to_string(cs) && (any_sweep_size(c->any, true, 1, cs) || any_sweep_size(c->any, false, 1, cs))) {
+                c->sweep = cs;
+                return 0;
+            }
+    if (n == "default") {
+        set(fastN, c->r8_ok, c->r12_ok);
+        c->sweep = 0;
         return 0;
     }
     if (n == "register-64" && c->r8_ok) return set(fastN, 1, 0);
@@ -1610,7 +1614,8 @@ extern "C" int lfts_transform_radices(int n, int *radices, int cap, int *count) 
 
 extern "C" int lfts_step_impl(lfts_ctx c, char *name, size_t cap) {
     if (!c || !name || cap == 0) return fail("null argument");
-    std::string n = c->r8 ? (c->xcap ? "register-64 xcap" + std::to_string(c->xcap) : std::string("register-64"))
+    std::string n = c->sweep > 0 ? "cluster-" + std::to_string(c->sweep)
+                  : c->r8 ? (c->xcap ? "register-64 xcap" + std::to_string(c->xcap) : std::string("register-64"))
                   : c->r12 ? (c->xcap ? "register-96 xcap" + std::to_string(c->xcap) : std::string("register-96"))
                   : c->fastN ? std::string("cubic") : std::string("generic");
     std::strncpy(name, n.c_str(), cap - 1);
