@@ -168,11 +168,12 @@ int lfts_realspace_tables(lfts_ctx ctx, double b2, double ds, int dim, const dou
 int lfts_step_realspace(lfts_ctx ctx, const lfts_step_job *jobs, int njobs, int s, int dim);
 
 /* Step autotuner (no counterpart in the reference, whose cuFFT plans are fixed):
- * times lfts_step_continuous for every implementation this grid supports
- * (register-resident line transforms at 64^3 / 96^3 with their x-pass CTA
- * residencies, the compile-time cubic kernels, the generic mixed-radix
- * kernels) on njobs synthetic jobs, reps timed calls each, and makes the
- * fastest the context's step implementation (continuous and discrete).  The
+ * times sweeps of eight steps (lfts_sweep_continuous, as solvers run them) for
+ * every implementation this grid supports (register-resident line transforms at
+ * 64^3 / 96^3 with their x-pass CTA residencies, the compile-time cubic kernels,
+ * the generic kernels, in clusters where the default rule has them) on njobs
+ * synthetic jobs, reps timed calls each, and makes the fastest the context's step
+ * implementation (continuous and discrete), in place of one set by name.  The
  * most specialised one stays unless another is more than 5 % faster.  It
  * allocates and frees its own buffers, synchronises, and must not run inside a
  * graph capture.  report (may be NULL) receives the timings and the choice. */

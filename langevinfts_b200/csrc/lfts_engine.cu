@@ -1448,8 +1448,9 @@ extern "C" int lfts_dots_static(int precision, long long M, const lfts_dot_job *
 }
 
 // ---------------------------------------------------------------- autotuner
-// Times lfts_step_continuous for every step family the grid supports, and the
-// persistent x-pass residency of the register families, on njobs synthetic
+// Times sweeps (lfts_sweep_continuous, what a solver runs: seams between steps, or a
+// cluster launch where the rule has one) for every step family the grid supports, and
+// the persistent x-pass residency of the register families, on njobs synthetic
 // jobs (q = 1, fac = 1, bond tables of a box of edge n), and keeps the fastest.
 // The most specialised family (register-resident, then cubic, then generic) is
 // the default; another one is taken only when it is more than 5 % faster, so
@@ -1465,7 +1466,8 @@ extern "C" int lfts_autotune(lfts_ctx c, int njobs, int reps, char *report, size
     if (!c) return fail("null context");
     if (njobs < 1 || njobs > 65535) return fail("autotune: njobs must be 1..65535");
     if (reps < 1) reps = 5;
-    const int fastN = c->fastN, r8v = c->r8, r12v = c->r12, xcap0 = c->xcap;
+    const int fastN = c->fastN, r8v = c->r8, r12v = c->r12, xcap0 = c->xcap, sweep0 = c->sweep;
+    constexpr int STEPS = 8;  // a sweep
     std::vector<TuneCand> cands;
     if (r8v) {
         cands.push_back({fastN, 1, 0, 0, "register-64"});
@@ -1528,19 +1530,21 @@ extern "C" int lfts_autotune(lfts_ctx c, int njobs, int reps, char *report, size
         CK(cudaMemcpy(djobs, hj.data(), sizeof(lfts_step_job) * njobs, cudaMemcpyHostToDevice));
     }
     std::vector<float> ms(cands.size(), 0.f);
+    c->sweep = 0;
+    // strides of zero: every step writes the same slice, and only the times matter
     for (size_t k = 0; k < cands.size() && rc == 0; k++) {
         c->fastN = cands[k].fastN;
         c->r8 = cands[k].r8;
         c->r12 = cands[k].r12;
         c->xcap = cands[k].xcap;
-        for (int i = 0; i < 2 && rc == 0; i++) rc = lfts_step_continuous(c, djobs, njobs, 0);
+        for (int i = 0; i < 2 && rc == 0; i++) rc = lfts_sweep_continuous(c, djobs, njobs, 0, STEPS);
         if (rc) break;
         CK(cudaEventRecord(e0, c->stream));
-        for (int i = 0; i < reps && rc == 0; i++) rc = lfts_step_continuous(c, djobs, njobs, 0);
+        for (int i = 0; i < reps && rc == 0; i++) rc = lfts_sweep_continuous(c, djobs, njobs, 0, STEPS);
         CK(cudaEventRecord(e1, c->stream));
         CK(cudaEventSynchronize(e1));
         CK(cudaEventElapsedTime(&ms[k], e0, e1));
-        ms[k] /= (float)reps;
+        ms[k] /= (float)(reps * STEPS);
     }
     if (rc == 0) rc = check_kernel_errors();
     if (rc == 0) {
@@ -1562,6 +1566,7 @@ extern "C" int lfts_autotune(lfts_ctx c, int njobs, int reps, char *report, size
         c->r8 = r8v;
         c->r12 = r12v;
         c->xcap = xcap0;
+        c->sweep = sweep0;
     }
     cleanup();
     if (report && report_cap) {
