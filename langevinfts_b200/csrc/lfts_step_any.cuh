@@ -90,10 +90,12 @@ __device__ __forceinline__ Point point_at(const Plan &g, int i, const short *iy,
     return {p, iy[yr], iz[c], r * g.pitch + c};
 }
 
-// v / 3 as a product and one correction (a quotient of FP64 numbers costs ten times this)
+// v / 3 as v times a third in two parts (a quotient of FP64 numbers costs ten times
+// this).  Both parts are positive: an infinite v stays infinite.
 template <typename T> __device__ __forceinline__ T third(T v) {
-    const T r = (T)(1.0 / 3.0), y = v * r;
-    return y + (v - (T)3 * y) * r;
+    constexpr T hi = sizeof(T) == 8 ? (T)0x1.5555555555555p-2 : (T)0x1.555554p-2;  // a third, rounded down
+    constexpr T lo = sizeof(T) == 8 ? (T)(1.0 / 3.0 * 0x1p-54) : (T)(1.0 / 3.0 - (double)hi);
+    return fma(v, hi, v * lo);
 }
 
 constexpr int U = 4;  // independent global loads a thread keeps in flight
