@@ -576,8 +576,17 @@ static int bond_tables_t(lfts_ctx c, double b2, double ds, const double *lx, voi
     CK(cudaStreamSynchronize(c->stream));
     return 0;
 }
+// Tables are written by kernels: a host address, which a copy to the device would
+// refuse, has to be refused before the launch.
+static int check_table(const void *p, const char *what) {
+    cudaPointerAttributes at;
+    CK(cudaPointerGetAttributes(&at, p));
+    if (at.type == cudaMemoryTypeUnregistered) return fail(std::string(what) + ": the output must be device memory");
+    return 0;
+}
 extern "C" int lfts_bond_tables(lfts_ctx c, double b2, double ds, const double *lx, void *b_out, void *bh_out) {
     if (!c || !lx || !b_out || !bh_out) return fail("null argument");
+    if (check_table(b_out, "lfts_bond_tables") || check_table(bh_out, "lfts_bond_tables")) return -1;
     return c->prec == 8 ? bond_tables_t<double>(c, b2, ds, lx, b_out, bh_out)
                         : bond_tables_t<float>(c, b2, ds, lx, b_out, bh_out);
 }
@@ -585,6 +594,7 @@ extern "C" int lfts_bond_tables(lfts_ctx c, double b2, double ds, const double *
 // Pseudo.cpp:84-153: k_d^2 (2 pi / L_d)^2, doubled for 0 < kz < n2/2
 extern "C" int lfts_fourier_basis(lfts_ctx c, const double *lx, double *basis_out) {
     if (!c || !lx || !basis_out) return fail("null argument");
+    if (check_table(basis_out, "lfts_fourier_basis")) return -1;
     const GridPlan &g = c->g;
     const int tn[3] = {g.n0, g.n1, g.n2};
     double tdx[3] = {1.0, 1.0, 1.0};
