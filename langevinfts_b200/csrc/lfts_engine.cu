@@ -1723,7 +1723,7 @@ extern "C" int lfts_realspace_tables(lfts_ctx c, double b2, double ds, int dim, 
     return 0;
 }
 
-// 32 lines a block while the tile leaves room for two blocks on an SM (n <= 330), else 16
+// 32 lines a block while the tile leaves room for two blocks on an SM (n <= 361), else 16
 template <int DIM, int A, bool FIRST, bool LAST>
 static int rs_sweep(lfts_ctx c, const lfts_step_job *jobs, int nj, int s, int src_half) {
     const int n = A == 0 ? c->g.n0 : A == 1 ? c->g.n1 : c->g.n2;

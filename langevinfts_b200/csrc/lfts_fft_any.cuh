@@ -10,8 +10,8 @@
 // What bounds these transforms on the grids that use them is the number of
 // stages (each a shared-memory round trip and a barrier) and, with extents
 // known only at run time, the index arithmetic.  Hence
-//   * radices up to 16 (and 7, 9, 11, 13) in registers, so that every extent
-//     up to 256 with factors up to 13 takes two stages, most take no third;
+//   * radices up to 13 and 16 in registers: of the 112 extents from 2 to 256 with
+//     factors up to 13, 78 take one or two stages and 34 (75, 98, 105, 125 ...) three;
 //   * divisions by run-time extents as one multiply-high with a factor the
 //     host prepared, and twiddle indices that need no remainder;
 //   * lines vary fastest over threads, with an odd pitch between rows, so the

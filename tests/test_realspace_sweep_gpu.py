@@ -1,6 +1,8 @@
 """The tiled real-space sweeps at the edges of their tiles: fewer lines than a
-tile, one line more, axes of one and two points, and an axis long enough for the
-narrow tile.  Against the numpy restatement, to round-off per step."""
+tile, one line more, axes of two points (the fewest a box may have) with every wall,
+and along each axis an extent above 361, where the tile has 16 lines instead of 32,
+with line counts that 16 does not divide.  Against the numpy restatement, to round-off
+per step."""
 import ctypes as C
 
 import numpy as np
@@ -13,6 +15,10 @@ CASES = [([5, 4, 3], ["periodic"] * 6), ([3, 11, 33], ["periodic", "periodic", "
          ([40, 6, 7], ["absorbing", "reflecting", "periodic", "periodic", "reflecting", "reflecting"]),
          ([33, 3], ["periodic"] * 4), ([12, 340], ["periodic", "periodic", "absorbing", "absorbing"]), ([350, 5], ["reflecting"] * 4),
          ([17], ["periodic"] * 2), ([700], ["reflecting", "absorbing"]), ([4, 3, 360], ["periodic"] * 6)]
+P, R, A = ["periodic"] * 2, ["reflecting", "absorbing"], ["absorbing", "reflecting"]
+CASES += [([361, 17], P + R), ([363, 17], P + R), ([370, 19], R + P), ([19, 370], P + A), ([4, 5, 370], P + R + A), ([370, 3, 7], R + P + P),
+          ([3, 370, 6], A + R + P), ([500], P)]
+CASES += [([2], P), ([2], R), ([2, 2], P + A), ([2, 33], R + P), ([2, 2, 2], P + R + A), ([5, 2, 3], A + P + R), ([3, 17, 2], P + P + P)]
 
 
 @pytest.mark.parametrize("nx,bc", CASES, ids=lambda v: "x".join(map(str, v)) if isinstance(v[0], int) else v[-1])
