@@ -898,6 +898,14 @@ def roofline_step_kernel(nx, njobs, reps=20, prec=8, impl=None):
     ev[1].record(stream)
     ev[1].synchronize()
     ms = ev[0].elapsed_time(ev[1]) / reps
+    # the same steps in sweeps of eight, as solvers run them: one kernel at each seam between two
+    check(ctx.lib.lfts_sweep_continuous(ctx.h, jp, njobs, 0, 8))
+    ev[0].record(stream)
+    for _ in range((reps + 7) // 8):
+        check(ctx.lib.lfts_sweep_continuous(ctx.h, jp, njobs, 0, 8))
+    ev[1].record(stream)
+    ev[1].synchronize()
+    roofline_step_kernel.sweep_ms = ev[0].elapsed_time(ev[1]) / (8 * ((reps + 7) // 8))
     ctx.close()
     roofline_step_kernel.impl = name.value.decode()
     return ms, M, Mc
@@ -1060,7 +1068,7 @@ def run_ours(args):
         "gpu_launches": int(launches),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "kernel": "lfts_step_continuous (5 fused FFT-pass kernels)",
-                     "launch_ms": ms, "jobs_per_launch": njobs,
+                     "launch_ms": ms, "sweep_step_ms": roofline_step_kernel.sweep_ms, "jobs_per_launch": njobs,
                      "bytes_model": f"{s_bytes}*(12M+24Mc) per job (pass model), peak = measured hbm_gbs",
                      "traffic_source": "ncu dram bytes per job-step captured one kernel at a time at 32 jobs "
                                        "(profiles/step_continuous_64cubed.txt) x jobs per launch; at 128 jobs L2 "

@@ -839,8 +839,9 @@ extern "C" int lfts_step_discrete(lfts_ctx c, const lfts_step_job *jobs, int nj,
 }
 
 // ---------------------------------------------------------------- sweeps
-// CTAs per job of a cluster sweep, 0 for step by step.  The cubic and register families
-// keep their grids: 22 us a step at 32^3 FP64 against 32 in clusters of 16, 19 against 19 at 16^3.
+// CTAs per job of a cluster sweep, 0 for separate launches.  The cubic and register families
+// keep their grids: FP64, 2 jobs, 19.1 us a step at 32^3 against 32.4 in clusters of 16, 14.2
+// against 19.3 at 16^3 (with 64 jobs there 31 against 24 in clusters of 8: not ruled for).
 static int sweep_size(lfts_ctx c, bool continuous, int nj) {
     if (!c->any || c->sweep < 0 || (c->sweep == 0 && c->fastN)) return 0;
     return any_sweep_size(c->any, continuous, nj, c->sweep);

@@ -370,11 +370,13 @@ void any_xstress(const AnyGrid *a, cudaStream_t st, const lfts_step_job *sj, con
     a->prec == 8 ? xstress<double>(a, st, sj, jobs, nj, basis, partials) : xstress<float>(a, st, sj, jobs, nj, basis, partials);
 }
 // A sweep's step costs barriers and transposes whatever the grid, then time per point
-// a CTA holds; the separate passes cost five (discrete: three) launches, then time per
-// point of all jobs.  Microseconds measured on a B200, FP64 (FP32): 84 x 48, 2 jobs 20.3 a
-// step in clusters of 16 against 27.7 (17.7 / 27.9); 256 points 16.2 / 25.4; 24^3 25 / 30;
-// 32^3, 32 768 points, 32.5 / 32.0 (26.6 / 30.4): the lines cross near 1500 (2500) points a
-// CTA.  More clusters than the device holds at once run in waves.
+// a CTA holds; the separate passes cost four (discrete: two) launches, then time per
+// point of all jobs.  Microseconds a step measured on a B200, 2 jobs, FP64 (FP32), clusters
+// of 16 / separate: 84 x 48 20.6 / 26.8 (17.7 / 27.0); 256 points 16.5 / 25.0 (14.2 / 22.9);
+// 24^3 25.0 / 27.8 (21.5 / 27.1); 32^3, 32 768 points, 32.4 / 30.2 (26.8 / 28.3): the lines
+// cross near 1500 (2500) points a CTA.  More clusters than the device holds at once run in
+// waves.  Where the rule misses the best of the sizes it is by up to a quarter, with many
+// jobs on one short axis (256 points, 64 jobs: clusters of 8 19.7, of 2 16.5).
 int any_sweep_size(const AnyGrid *a, bool continuous, int nj, int force) {
     const int *res = continuous ? a->clusters_cont : a->clusters_disc;
     if (force) {
